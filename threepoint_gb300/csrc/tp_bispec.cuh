@@ -9,6 +9,7 @@
 #pragma once
 #include <type_traits>
 
+#include "tp_bispec64.cuh"
 #include "tp_internal.cuh"
 
 namespace tp {
@@ -40,9 +41,18 @@ struct Mth<double> {
   static __device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
 };
 
+// integer-arithmetic rows of the FP64 integrands (tp_bispec64.cuh)
+template <typename R>
+struct CosmoI64 {};
+template <>
+struct CosmoI64<double> {
+  const Node64* n64 = nullptr;  // [NNODE]
+  Cosmo64 c64 = {nullptr, 0, 0.0, 0.0, 0, 0};
+};
+
 // Cosmology constants of the integrands in arithmetic type R.
 template <typename R>
-struct CosmoK {
+struct CosmoK : CosmoI64<R> {
   R omh2, sa, one_m_sa, sh043, theta2, l2theta2, c184, ehc, ns, alpha_max;
   R l2h;             // log2(h)
   R h;
@@ -268,6 +278,76 @@ __device__ __forceinline__ R bispec_node(const R* __restrict__ nc, int j, const 
     return row[NC_W] * bispec_eval<R>(row, 1, row[NC_S], row[NC_L2S], row[NC_HF], row[NC_L2HF], T, K);
   }
 }
+
+// Kahan accumulator
+template <typename R>
+struct KSum {
+  R s = 0, c = 0;
+  __device__ __forceinline__ void add(R v) {
+    R y = v - c;
+    R t = s + y;
+    c = (t - s) - y;
+    s = t;
+  }
+};
+template <>
+struct KSum<double> {
+  double s = 0;
+  __device__ __forceinline__ void add(double v) { s += v; }
+};
+
+// ---------------------------------------------------------------------------
+// FP64 point path in integer arithmetic (tp_bispec64.cuh)
+#if defined(__CUDACC__)
+// F2_tree of the three pairs as make_tri forms them. The rounding of the
+// differences of squares is amplified by (l_max / l_min)^2, so it is compiled
+// where nothing else of its caller can be contracted into it.
+static __device__ __noinline__ void f2_trees(double l1, double l2, double l3, double* f2t) {
+  f2t[0] = f2_tree(l1, l2, l3);
+  f2t[1] = f2_tree(l2, l3, l1);
+  f2t[2] = f2_tree(l3, l1, l2);
+}
+
+// false (T.ok = 0) where the triangle or the cosmology is outside its domain
+__device__ __forceinline__ bool tri64_record(double l1, double l2, double l3, const CosmoK<double>& K, Tri64& T) {
+  double f2t[3];
+  f2_trees(l1, l2, l3, f2t);
+  const bool ok = K.c64.ok && tri64_make(l1, l2, l3, f2t, K.c64.lo, K.c64.hi, d_i64tab, T);
+  T.ok = ok;
+  return ok;
+}
+
+// sum of W B over nodes j0 .. j0 + nj - 1 with the FP64 instructions; rows NC_*
+static __device__ __noinline__ double bkappa_nodes_f64(const double* nc, int j0, int nj, const Tri<double>& T,
+                                                       const CosmoK<double>& K) {
+  KSum<double> acc;
+  for (int j = j0; j < j0 + nj; ++j) {
+    double v = bispec_node<double>(nc, j, T, K);
+    if (v != v) v = 0;  // NaN in bispec -> 0 (bispectrum.cu:327-331)
+    acc.add(v);
+  }
+  return acc.s;
+}
+
+__device__ __forceinline__ double bkappa64_nodes(const Node64* __restrict__ rows, const double* nc, int j0, int nj,
+                                                 const Tri64& T, const CosmoK<double>& K,
+                                                 const uint64_t* __restrict__ ex2) {
+  double s = 0;
+  for (int j = j0; j < j0 + nj; ++j) {
+    const Node64& N = rows[j];
+    double v;
+    if (N.ok) {
+      v = N.w * bispec64(N, T, K.c64, ex2);
+    } else {
+      Tri<double> D;
+      make_tri<double>(sf_to({T.s[0].m, T.s[0].e}), sf_to({T.s[1].m, T.s[1].e}), sf_to({T.s[2].m, T.s[2].e}), D);
+      v = bkappa_nodes_f64(nc, j, 1, D, K);
+    }
+    if (v == v) s += v;
+  }
+  return s;
+}
+#endif
 
 // ---------------------------------------------------------------------------
 // FP32 point path of <Map^3> and b_kappa: NF_* node rows (tp_internal.cuh).
@@ -720,22 +800,5 @@ __device__ __forceinline__ double uhat(double eta) {
   double t = 0.5 * eta * eta;
   return t * exp(-t);
 }
-
-// Kahan accumulator
-template <typename R>
-struct KSum {
-  R s = 0, c = 0;
-  __device__ __forceinline__ void add(R v) {
-    R y = v - c;
-    R t = s + y;
-    c = (t - s) - y;
-    s = t;
-  }
-};
-template <>
-struct KSum<double> {
-  double s = 0;
-  __device__ __forceinline__ void add(double v) { s += v; }
-};
 
 }  // namespace tp

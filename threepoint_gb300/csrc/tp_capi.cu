@@ -299,6 +299,8 @@ void tp_ctx::free_cosmo() {
   cudaFree(d_ck32);
   cudaFree(d_plt);
   cudaFree(d_ehg);
+  cudaFree(d_n64);
+  cudaFree(d_p64);
   cudaFree(d_halo);
   d_halo = nullptr;
   halo_ready.clear();
@@ -316,6 +318,8 @@ void tp_ctx::free_cosmo() {
   d_ck32 = nullptr;
   d_plt = nullptr;
   d_ehg = nullptr;
+  d_n64 = nullptr;
+  d_p64 = nullptr;
   n_cosmo = 0;
   cosmo_cap = 0;
   nz_cap = 0;
@@ -446,6 +450,8 @@ extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n,
     if (e == cudaSuccess) e = dalloc((CosmoK<float>**)&ctx->d_ck32, cap);
     if (e == cudaSuccess) e = dalloc(&ctx->d_plt, (size_t)cap * PLT_N);
     if (e == cudaSuccess) e = dalloc(&ctx->d_ehg, (size_t)cap * EHG_N);
+    if (e == cudaSuccess) e = dalloc(&ctx->d_n64, (size_t)cap * NNODE);
+    if (e == cudaSuccess) e = dalloc(&ctx->d_p64, (size_t)cap * P64_N);
     if (e != cudaSuccess) {
       ctx->free_cosmo();
       return tp_cuda(ctx, e, "cosmology allocation");
@@ -466,7 +472,8 @@ extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n,
   if (e == cudaSuccess)
     e = build_tables(ctx->d_cos, ctx->d_eh, ctx->d_nz, nz_stride, ctx->d_tab, ctx->d_ncoef64, ctx->d_ncoef32,
                      ctx->d_fcoef32, ctx->d_hcoef, ctx->d_hcoef32, ctx->d_wscale64, ctx->d_wscale32, (CosmoK<double>*)ctx->d_ck64,
-                     (CosmoK<float>*)ctx->d_ck32, ctx->d_plt, ctx->d_ehg, n, s);
+                     (CosmoK<float>*)ctx->d_ck32, ctx->d_plt, ctx->d_ehg,
+                     ctx->d_n64, ctx->d_p64, n, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return tp_cuda(ctx, e, "table build");
   return TP_OK;

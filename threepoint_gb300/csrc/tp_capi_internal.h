@@ -7,6 +7,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "tp_bispec64.cuh"
 #include "tp_internal.cuh"
 
 // NVTX range over one entry-point call (host time: the table build, the
@@ -49,6 +50,9 @@ struct tp_ctx {
   void* d_ck64 = nullptr;
   void* d_ck32 = nullptr;
   float4* d_plt = nullptr;  // [n_cosmo][PLT_N] log2 P_lin cubic segments
+  // integer-arithmetic forms of the FP64 integrands (tp_bispec64.cuh)
+  tp::Node64* d_n64 = nullptr;   // [n_cosmo][NNODE]
+  tp::P64Cell* d_p64 = nullptr;  // [n_cosmo][P64_N]
   double* d_ehg = nullptr;  // [n_cosmo][EHG_N] 2 ln T(k) of the sigma(R) integrand
   // halo-model tables (covariance terms T5-T7), built per cosmology on first use
   tp::HaloTab* d_halo = nullptr;

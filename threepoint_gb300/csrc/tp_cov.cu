@@ -204,17 +204,22 @@ template <typename R>
 struct BkProd {
   static constexpr int G = 16;  // 2 b_kappa x 8 node chunks
   static constexpr int PD = 1;
-  static constexpr int MINB = 1;
+  static constexpr int MINB = sizeof(R) == 8 ? 2 : 1;
   static constexpr bool CLUSTER16 = false;
   static constexpr int NS = 2;
   __device__ static int slot(int g) { return g >> 3; }
-  static constexpr int CH = 4;
+  // FP64: one region per chunk (93 points of 432-byte records), so that two
+  // CTAs share an SM
+  static constexpr int CH = sizeof(R) == 8 ? 1 : 4;
   // FP64 rows NC_* with Tri<double>; FP32 rows NF_* (pair-interleaved, packed
   // node pairs as in k_map3) with TriF
   struct RecD {
-    Tri<double> t[2];
+    union {
+      Tri64 t[2];
+      Tri<double> f64[2];  // of the FP64 instructions (f64form)
+    };
     double wt;
-    int valid;
+    int valid, f64form;
   };
   struct RecF {
     TriF t[2];
@@ -224,7 +229,11 @@ struct BkProd {
   typedef typename std::conditional<sizeof(R) == 4, RecF, RecD>::type Rec;
   static constexpr int REC = (int)sizeof(Rec);
   const int* job_order = nullptr;
-  static constexpr size_t PSMEM = sizeof(R) * NCP * NNODE + sizeof(CosmoK<R>) + 64;
+  static constexpr bool REF = sizeof(R) == 8;  // FP64 instructions beside the integer form
+  int ref;
+  static constexpr size_t NODE_BYTES = sizeof(R) == 4 ? sizeof(R) * NCP * NNODE : sizeof(Node64) * NNODE;
+  static constexpr size_t EX2_BYTES = sizeof(R) == 4 ? 0 : sizeof(I64Tables::ex2);
+  static constexpr size_t PSMEM = NODE_BYTES + EX2_BYTES + sizeof(CosmoK<R>) + 64;
 
   const CovJob* jobs;
   const R* ncoef;  // NC_* rows (FP64) or NF_* rows (FP32) of the cosmology
@@ -241,7 +250,13 @@ struct BkProd {
     s_nc = (R*)psmem;
     if (!loaded) {
       __syncthreads();
-      for (int i = threadIdx.x; i < NCP * NNODE; i += blockDim.x) s_nc[i] = ncoef[i];
+      const uint32_t* src = (const uint32_t*)(const void*)ncoef;
+      if constexpr (sizeof(R) == 8) {
+        src = (const uint32_t*)(const void*)ck.n64;
+        uint64_t* ex = (uint64_t*)(psmem + NODE_BYTES);
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) ex[i] = d_i64tab.ex2[i];
+      }
+      for (int i = threadIdx.x; i < (int)(NODE_BYTES / 4); i += blockDim.x) ((uint32_t*)psmem)[i] = src[i];
       __syncthreads();
       loaded = 1;
     }
@@ -259,9 +274,36 @@ struct BkProd {
 
   __device__ bool is_live(const char* r) const { return ((const Rec*)r)->valid != 0; }
 
+  // the reference form's point (FP64; see Map3Policy::setup_f64)
+  static __device__ __noinline__ bool setup_f64(const double* x, const double* th, double lmax, RecD& r) {
+    double l1 = exp(x[0]), l2 = exp(x[1]), l5 = exp(x[2]), c1 = cos(x[3]), c2 = cos(x[4]);
+    double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * c1);
+    double l6 = sqrt(l1 * l1 + l5 * l5 + 2 * l1 * l5 * c2);
+    bool zero = l3 > lmax || l6 > lmax || !(l3 > 0) || !(l6 > 0);
+    // b_kappa's own cut-offs (bispectrum.cu:295-296,315-318)
+    zero = zero || !(l3 > 1e-10) || !(l6 > 1e-10);
+    double wt = 0;
+    if (!zero) {
+      double lp = l1 * l2 * l5;
+      wt = uhat(l1 * th[0]) * uhat(l2 * th[1]) * uhat(l3 * th[2]) * uhat(l1 * th[3]) * uhat(l5 * th[4]) *
+           uhat(l6 * th[5]) * lp * lp;
+    }
+    r.valid = !zero && wt != 0.0;
+    r.wt = wt;
+    r.f64form = 1;
+    if (r.valid) {
+      make_tri<double>(l1, l2, l3, r.f64[0]);
+      make_tri<double>(l1, l5, l6, r.f64[1]);
+    }
+    return r.valid;
+  }
+
   __device__ bool setup(int p, const double* x, char* recp) {
     (void)p;
     Rec& r = *(Rec*)recp;
+    if constexpr (sizeof(R) == 8) {
+      if (ref || !ck.c64.ok) return setup_f64(x, th, lmax, r);
+    }
     double l1 = exp(x[0]), l2 = exp(x[1]), l5 = exp(x[2]), c1 = cos(x[3]), c2 = cos(x[4]);
     double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * c1);
     double l6 = sqrt(l1 * l1 + l5 * l5 + 2 * l1 * l5 * c2);
@@ -284,8 +326,9 @@ struct BkProd {
         make_tri<float>(l1, l5, l6, t);
         trif_from_tri(t, r.t[1]);
       } else {
-        make_tri<R>(l1, l2, l3, r.t[0]);
-        make_tri<R>(l1, l5, l6, r.t[1]);
+        r.f64form = 0;
+        if (!tri64_record(l1, l2, l3, ck, r.t[0]) || !tri64_record(l1, l5, l6, ck, r.t[1]))
+          setup_f64(x, th, lmax, r);
       }
     }
     return r.valid;
@@ -323,14 +366,9 @@ struct BkProd {
       }
       pv[0] = (double)(sm.x + sm.y);
     } else {
-      KSum<R> acc;
-#pragma unroll 2
-      for (int j = j0; j < j0 + 12; ++j) {
-        R v = bispec_node<R>(s_nc, j, r.t[i], ck);
-        if (v != v) v = (R)0;
-        acc.add(v);
-      }
-      pv[0] = (double)acc.s;
+      pv[0] = r.f64form ? bkappa_nodes_f64(ncoef, j0, 12, r.f64[i], ck)
+                        : bkappa64_nodes((const Node64*)s_nc, ncoef, j0, 12, r.t[i], ck,
+                                         (const uint64_t*)((const char*)s_nc + NODE_BYTES));
     }
   }
 

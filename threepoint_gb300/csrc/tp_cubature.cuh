@@ -25,6 +25,8 @@
 #include <cooperative_groups.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "tp_internal.cuh"
 
 namespace tp {
@@ -72,6 +74,19 @@ struct EngineCfg {
   int max_sweeps;
 };
 
+// Policies with P::REF: the region's axis, its values come from the reference
+// form of the integrand; its two largest fourth differences tie
+constexpr int SPLIT_AXIS = 7, SPLIT_AXIS_REF = 32, SPLIT_REF = 64, SPLIT_TIE = 128;
+
+template <class P, class = void>
+struct EngineRef {
+  static constexpr bool value = false;
+};
+template <class P>
+struct EngineRef<P, std::enable_if_t<P::REF>> {
+  static constexpr bool value = true;
+};
+
 // per-CTA region store
 template <int DIM, int FDIM>
 struct Slot {
@@ -82,7 +97,7 @@ struct Slot {
   double* err;    // [FDIM][cap]
   double* emax;   // [cap]
   int* pend;      // [cap]
-  uint8_t* split; // [cap]
+  uint8_t* split; // [cap] axis | SPLIT_*
   int cap;
   __host__ __device__ static constexpr size_t bytes(int cap) {
     return (size_t)cap * (sizeof(double) * (2 * DIM + 2 + 2 * FDIM) + sizeof(int) + 1) + 256;
@@ -149,6 +164,43 @@ __device__ inline void rule_point(int p, const double* c, const double* h, doubl
       x[d] = ((gray >> d) & 1) ? c[d] - r : c[d] + r;
     }
   }
+}
+
+// relative difference below which two errors (or fourth differences) count as
+// a tie of mirror-image regions (axes) that rounding decides: rounding moves
+// them by up to ~1e-9, and unrelated regions come this close with a
+// probability of ~1e-4 per cut
+constexpr double TIE_REL = 1e-6;
+
+// axis of the largest fourth difference, from the centre and the 4 DIM axis
+// points (the rule's first points); tie: another axis comes within TIE_REL
+template <int DIM, int FDIM>
+__device__ inline void rule_axis(const double* f, int* split, bool* split_tie) {
+  double diff[DIM];
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) diff[d] = 0;
+  for (int k = 0; k < FDIM; ++k) {
+    auto V = [&](int i) { return f[i * FDIM + k]; };
+    double val0 = V(0);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      double v0 = V(1 + 4 * d), v1 = V(2 + 4 * d), v2 = V(3 + 4 * d), v3 = V(4 + 4 * d);
+      diff[d] += fabs(v0 + v1 - 2 * val0 - GM::ratio * (v2 + v3 - 2 * val0));
+    }
+  }
+  double md = 0;
+  int dm = 0;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+    if (diff[d] > md) {
+      md = diff[d];
+      dm = d;
+    }
+  *split = dm;
+  *split_tie = false;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d)
+    if (d != dm && diff[d] >= md * (1.0 - TIE_REL)) *split_tie = true;
 }
 
 // Apply the embedded rule to one region's NP point values (f[p*FDIM+k]).
@@ -246,6 +298,16 @@ __device__ inline void rule_combine(const double* f, double vol, double hw0, dou
   }
 }
 
+// rule_combine that also tells whether the axis is a tie
+template <int DIM, int FDIM>
+__device__ inline void rule_combine_ref(const double* f, double vol, double hw0, double* val, double* err, int* split,
+                                        bool* split_tie) {
+  rule_combine<DIM, FDIM>(f, vol, hw0, val, err, split);
+  *split_tie = false;
+  int sp;
+  if constexpr (DIM > 1) rule_axis<DIM, FDIM>(f, &sp, split_tie);
+}
+
 // ---------------------------------------------------------------------------
 // block-wide helpers
 template <int NT>
@@ -318,7 +380,7 @@ struct EngineShared {
   double V[FDIM], E[FDIM];
   unsigned long long q_above;
   unsigned long long prefix;
-  int job, nlive, npend, status, stop, ktot, sweeps;
+  int job, nlive, npend, status, stop, ktot, sweeps, ref, nband, nref, nfull;
   long long neval;
 };
 
@@ -342,6 +404,17 @@ __host__ __device__ constexpr size_t engine_smem_bytes() {
 //   __device__ void finalize(const char* rec, const double* sum /*FDIM*/, double* fval /*FDIM*/)
 //   __device__ void end_job(int job, const double* V, const double* E, long long neval, int status)
 //   static constexpr size_t PSMEM (policy shared bytes)
+//   static constexpr bool REF (optional): the policy has two forms of the
+//   integrand that agree to rounding, a fast one and the reference form
+//   (int ref: 0, or not for the reference form; set here). An integrand symmetric under an exchange or a
+//   reflection of its variables gives mirror-image regions whose errors differ
+//   only by rounding, and where a sweep's cut falls between them the reference
+//   form's rounding decides whether one or both are split (a bitwise tie splits
+//   both); likewise the axis of a region on the mirror plane. Those regions
+//   (errors within TIE_REL of the cut; splits with two equal fourth
+//   differences) are evaluated again with the reference form before the cut is
+//   drawn, so the region sequence, and with it the result to ~1e-15, is the
+//   reference form's.
 //
 // CS > 1 (launch with thread-block clusters of CS CTAs): the CTAs of a
 // cluster own one integral together. Every sweep's pending regions are dealt
@@ -367,10 +440,12 @@ template <int DIM, int FDIM, int NT, class P, int CS = 1>
 __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineCfg cfg, char* scratch,
                               size_t slot_bytes) {
   constexpr int NP = GMRule<DIM>::NP;
+  constexpr int NPAX = 1 + 4 * DIM;  // the rule's centre and axis points
   constexpr int CH = P::CH;
   constexpr int G = P::G;
   constexpr int PD = P::PD;  // values per group item (>= 1)
   constexpr int NS = P::NS;  // group classes: item g adds into sum class P::slot(g)
+  constexpr bool REF = EngineRef<P>::value;
   static_assert(P::CH * NP <= 1024, "live list holds one chunk");
   extern __shared__ __align__(16) char smem[];
   char* psmem = smem;
@@ -418,80 +493,200 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
       es->stop = 0;
       es->neval = 0;
       es->sweeps = 0;
+      es->ref = 0;
     }
     engine_cluster_sync<CS>();
 
-    for (int sweep = 0;; ++sweep) {
+    for (int sweep = 0;;) {
       // ---------------- evaluate the pending regions ----------------------
       const int npend = es0->npend;
-      // a cluster deals out chunks of CH regions, or single regions while a
-      // sweep has fewer than CS * CH of them (all ranks then have work)
-      const int step = (CS > 1 && npend < CS * CH) ? 1 : CH;
-      for (int base = crank * step; base < npend; base += CS * step) {
-        const int nreg = min(step, npend - base);
-        const int npts = nreg * NP;
-        // (a) point setup; points that need the expensive inner sums are
-        //     appended to a compact live list
-        for (int p = tid; p < npts; p += NT) {
-          int r = S.pend[base + p / NP];
-          double c[DIM], h[DIM], x[DIM];
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            c[d] = S.cen[(size_t)d * S.cap + r];
-            h[d] = S.hw[(size_t)d * S.cap + r];
-          }
-          rule_point<DIM>(p % NP, c, h, x);
-          if (pol.setup(p, x, recs + (size_t)p * P::REC)) es->live_list[atomicAdd(&es->nlive_chunk, 1)] = p;
-        }
-        __syncthreads();
-        // (b) (live point, group) items: equal-cost work for every thread
-        const int nl = es->nlive_chunk;
-        for (int it = tid; it < nl * G; it += NT) {
-          int g = it / nl, q = it - g * nl;
-          int p = es->live_list[q];
-          double pv[PD];
-          pol.group(recs + (size_t)p * P::REC, g, pv);
-#pragma unroll
-          for (int k = 0; k < PD; ++k) part[((size_t)g * npts + p) * PD + k] = pv[k];
-        }
-        __syncthreads();
-        // (c) per-point totals (fixed group order -> deterministic)
-        for (int p = tid; p < npts; p += NT) {
-          double s[NS * PD];
-#pragma unroll
-          for (int k = 0; k < NS * PD; ++k) s[k] = 0;
-          if (pol.is_live(recs + (size_t)p * P::REC))
-            for (int g = 0; g < G; ++g) {
-              const int sl = P::slot(g);
-#pragma unroll
-              for (int k = 0; k < PD; ++k) s[sl * PD + k] += part[((size_t)g * npts + p) * PD + k];
+      const int ref = REF ? es0->ref : 0;
+      if constexpr (REF) pol.ref = ref;
+      if constexpr (!REF) {
+        // a cluster deals out chunks of CH regions, or single regions while a
+        // sweep has fewer than CS * CH of them (all ranks then have work)
+        const int step = (CS > 1 && npend < CS * CH) ? 1 : CH;
+        for (int base = crank * step; base < npend; base += CS * step) {
+          const int nreg = min(step, npend - base);
+          const int npts = nreg * NP;
+          // (a) point setup; points that need the expensive inner sums are
+          //     appended to a compact live list
+          for (int p = tid; p < npts; p += NT) {
+            int r = S.pend[base + p / NP];
+            double c[DIM], h[DIM], x[DIM];
+  #pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              c[d] = S.cen[(size_t)d * S.cap + r];
+              h[d] = S.hw[(size_t)d * S.cap + r];
             }
-          pol.finalize(recs + (size_t)p * P::REC, s, fval + (size_t)p * FDIM);
-        }
-        if (tid == 0) es->nlive_chunk = 0;
-        __syncthreads();
-        for (int rr = tid; rr < nreg; rr += NT) {
-          int r = S.pend[base + rr];
-          double v[FDIM], e[FDIM];
-          int sp;
-          rule_combine<DIM, FDIM>(fval + (size_t)rr * NP * FDIM, S.vol[r], S.hw[r], v, e, &sp);
-          double em = 0;
-#pragma unroll
-          for (int k = 0; k < FDIM; ++k) {
-            S.val[(size_t)k * S.cap + r] = v[k];
-            S.err[(size_t)k * S.cap + r] = e[k];
-            em = fmax(em, e[k]);
+            rule_point<DIM>(p % NP, c, h, x);
+            if (pol.setup(p, x, recs + (size_t)p * P::REC)) es->live_list[atomicAdd(&es->nlive_chunk, 1)] = p;
           }
-          S.emax[r] = em;
-          S.split[r] = (uint8_t)sp;
+          __syncthreads();
+          // (b) (live point, group) items: equal-cost work for every thread
+          const int nl = es->nlive_chunk;
+          for (int it = tid; it < nl * G; it += NT) {
+            int g = it / nl, q = it - g * nl;
+            int p = es->live_list[q];
+            double pv[PD];
+            pol.group(recs + (size_t)p * P::REC, g, pv);
+  #pragma unroll
+            for (int k = 0; k < PD; ++k) part[((size_t)g * npts + p) * PD + k] = pv[k];
+          }
+          __syncthreads();
+          // (c) per-point totals (fixed group order -> deterministic)
+          for (int p = tid; p < npts; p += NT) {
+            double s[NS * PD];
+  #pragma unroll
+            for (int k = 0; k < NS * PD; ++k) s[k] = 0;
+            if (pol.is_live(recs + (size_t)p * P::REC))
+              for (int g = 0; g < G; ++g) {
+                const int sl = P::slot(g);
+  #pragma unroll
+                for (int k = 0; k < PD; ++k) s[sl * PD + k] += part[((size_t)g * npts + p) * PD + k];
+              }
+            pol.finalize(recs + (size_t)p * P::REC, s, fval + (size_t)p * FDIM);
+          }
+          if (tid == 0) es->nlive_chunk = 0;
+          __syncthreads();
+          for (int rr = tid; rr < nreg; rr += NT) {
+            int r = S.pend[base + rr];
+            double v[FDIM], e[FDIM];
+            int sp;
+            rule_combine<DIM, FDIM>(fval + (size_t)rr * NP * FDIM, S.vol[r], S.hw[r], v, e, &sp);
+            double em = 0;
+  #pragma unroll
+            for (int k = 0; k < FDIM; ++k) {
+              S.val[(size_t)k * S.cap + r] = v[k];
+              S.err[(size_t)k * S.cap + r] = e[k];
+              em = fmax(em, e[k]);
+            }
+            S.emax[r] = em;
+            S.split[r] = (uint8_t)sp;
+          }
+          __syncthreads();
         }
-        __syncthreads();
+      } else {
+        // as below; a reference pass deals its few regions out evenly and shares
+        // their items over the cluster's threads. Its first nfull regions take the
+        // whole rule, the others its axis points.
+        const int nfull = ref ? es0->nfull : npend;
+        const int step = CS == 1 ? CH : ref ? min(CH, (npend + CS - 1) / CS) : npend < CS * CH ? 1 : CH;
+        for (int base0 = 0; base0 < npend; base0 += CS * step) {
+          const int base = base0 + crank * step;
+          const int nreg = max(0, min(step, npend - base));
+          auto points = [&](int first, int n) {  // of regions first .. first + n - 1
+            const int nf = max(0, min(n, nfull - first));
+            return nf * NP + (n - nf) * NPAX;
+          };
+          const int npts = points(base, nreg), nf = max(0, min(nreg, nfull - base));
+          const bool shared = CS > 1 && ref;
+          if (!shared && nreg == 0) break;
+          // (a) point setup; points that need the expensive inner sums are
+          //     appended to a compact live list
+          for (int p = tid; p < npts; p += NT) {
+            const int pa = p - nf * NP;  // index among the axis points
+            int r = S.pend[base + (pa < 0 ? p / NP : nf + pa / NPAX)];
+            double c[DIM], h[DIM], x[DIM];
+  #pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              c[d] = S.cen[(size_t)d * S.cap + r];
+              h[d] = S.hw[(size_t)d * S.cap + r];
+            }
+            rule_point<DIM>(pa < 0 ? p % NP : pa % NPAX, c, h, x);
+            if (pol.setup(p, x, recs + (size_t)p * P::REC)) es->live_list[atomicAdd(&es->nlive_chunk, 1)] = p;
+          }
+          // (b) (live point, group) items: equal-cost work for every thread
+          if (!shared) {
+            __syncthreads();
+            const int nl = es->nlive_chunk;
+            for (int it = tid; it < nl * G; it += NT) {
+              int g = it / nl, q = it - g * nl;
+              int p = es->live_list[q];
+              double pv[PD];
+              pol.group(recs + (size_t)p * P::REC, g, pv);
+  #pragma unroll
+              for (int k = 0; k < PD; ++k) part[((size_t)g * npts + p) * PD + k] = pv[k];
+            }
+            __syncthreads();
+          }
+          if constexpr (CS > 1) {
+            if (shared) {
+              cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+              cl.sync();
+              // items of rank 0, then of rank 1, ...: records are copied and
+              // sums written through distributed shared memory
+              int first = 0;
+              for (int o = 0; o < CS && base0 + o * step < npend; ++o) {
+                EngineShared<FDIM>* eo = cl.map_shared_rank(es, o);
+                const char* ro = cl.map_shared_rank(recs, o);
+                double* po = cl.map_shared_rank(part, o);
+                const int no = points(base0 + o * step, min(step, npend - base0 - o * step)), nl = eo->nlive_chunk;
+                const int skip = (crank * NT + tid - first) % (CS * NT);
+                for (int it = skip < 0 ? skip + CS * NT : skip; it < nl * G; it += CS * NT) {
+                  int g = it / nl, q = it - g * nl;
+                  int p = eo->live_list[q];
+                  alignas(16) char rec[(P::REC + 15) & ~15];
+  #pragma unroll
+                  for (int w = 0; w < P::REC / 4; ++w)
+                    ((uint32_t*)rec)[w] = ((const uint32_t*)(ro + (size_t)p * P::REC))[w];
+                  double pv[PD];
+                  pol.group(rec, g, pv);
+  #pragma unroll
+                  for (int k = 0; k < PD; ++k) po[((size_t)g * no + p) * PD + k] = pv[k];
+                }
+                first += nl * G;
+              }
+              cl.sync();
+            }
+          }
+          // (c) per-point totals (fixed group order -> deterministic)
+          for (int p = tid; p < npts; p += NT) {
+            double s[NS * PD];
+  #pragma unroll
+            for (int k = 0; k < NS * PD; ++k) s[k] = 0;
+            if (pol.is_live(recs + (size_t)p * P::REC))
+              for (int g = 0; g < G; ++g) {
+                const int sl = P::slot(g);
+  #pragma unroll
+                for (int k = 0; k < PD; ++k) s[sl * PD + k] += part[((size_t)g * npts + p) * PD + k];
+              }
+            pol.finalize(recs + (size_t)p * P::REC, s, fval + (size_t)p * FDIM);
+          }
+          if (tid == 0) es->nlive_chunk = 0;
+          __syncthreads();
+          for (int rr = tid; rr < nreg; rr += NT) {
+            int r = S.pend[base + rr];
+            int sp;
+            bool tie;
+            if constexpr (DIM > 1) {
+              if (rr >= nf) {  // the axis alone
+                rule_axis<DIM, FDIM>(fval + (size_t)(nf * NP + (rr - nf) * NPAX) * FDIM, &sp, &tie);
+                S.split[r] = (uint8_t)((S.split[r] & SPLIT_REF) | SPLIT_AXIS_REF | sp);
+                continue;
+              }
+            }
+            double v[FDIM], e[FDIM];
+            rule_combine_ref<DIM, FDIM>(fval + (size_t)rr * NP * FDIM, S.vol[r], S.hw[r], v, e, &sp, &tie);
+            sp |= ref ? SPLIT_REF | SPLIT_AXIS_REF : tie ? SPLIT_TIE : 0;
+            double em = 0;
+  #pragma unroll
+            for (int k = 0; k < FDIM; ++k) {
+              S.val[(size_t)k * S.cap + r] = v[k];
+              S.err[(size_t)k * S.cap + r] = e[k];
+              em = fmax(em, e[k]);
+            }
+            S.emax[r] = em;
+            S.split[r] = (uint8_t)sp;
+          }
+          __syncthreads();
+        }
       }
       if constexpr (CS > 1) engine_cluster_sync<CS>();
       // rank 0: totals, convergence, selection and splitting; a stop sets
       // es->stop and leaves this block
       if (crank == 0) do {
-      if (tid == 0) es->neval += (long long)npend * NP;
+      if (tid == 0 && !ref) es->neval += (long long)npend * NP;
 
       // ---------------- totals and convergence ----------------------------
       const int nlive = es->nlive;
@@ -614,6 +809,45 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
       }
       const unsigned long long tau = es->prefix;
 
+      // ---------------- ties that the reference form decides --------------
+      if constexpr (REF) {
+        if (!ref && tau != 0ull) {
+          const double kt = __longlong_as_double((long long)tau);
+          const double b0 = kt * (1.0 - TIE_REL), b1 = kt * (1.0 + TIE_REL);
+          if (tid == 0) es->nband = es->nref = 0;
+          __syncthreads();
+          // regions at the cut, where there is more than one
+          int nb = 0;
+          for (int i = tid; i < nlive; i += NT) nb += S.emax[i] >= b0 && S.emax[i] <= b1;
+          if (nb) atomicAdd(&es->nband, nb);
+          __syncthreads();
+          const bool band = es->nband > 1;
+          if (band) {
+            for (int i = tid; i < nlive; i += NT)
+              if (!(S.split[i] & SPLIT_REF) && S.emax[i] >= b0 && S.emax[i] <= b1)
+                S.pend[atomicAdd(&es->nref, 1)] = i;
+          }
+          __syncthreads();
+          const int nfl = es->nref;
+          __syncthreads();
+          // axes of the regions above them
+          for (int i = tid; i < nlive; i += NT)
+            if ((S.split[i] & (SPLIT_TIE | SPLIT_AXIS_REF)) == SPLIT_TIE && S.emax[i] >= (band ? b0 : kt) &&
+                !(band && S.emax[i] <= b1))
+              S.pend[atomicAdd(&es->nref, 1)] = i;
+          __syncthreads();
+          if (es->nref > 0) {
+            if (tid == 0) {
+              es->npend = es->nref;
+              es->nfull = nfl;
+              es->ref = 1;
+            }
+            __syncthreads();
+            break;  // all ranks evaluate them, then the cut is drawn again
+          }
+        }
+      }
+
       // ---------------- compaction: split every region with key >= tau ----
       const int chunk = (nlive + NT - 1) / NT;
       const int lo = min(tid * chunk, nlive), hi = min(lo + chunk, nlive);
@@ -638,7 +872,7 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
       for (int i = lo; i < hi; ++i) {
         if ((unsigned long long)__double_as_longlong(S.emax[i]) < tau) continue;
         const int u = nlive + rank;
-        const int d = S.split[i];
+        const int d = S.split[i] & SPLIT_AXIS;
         double v = 1;
 #pragma unroll
         for (int q = 0; q < DIM; ++q) {
@@ -665,10 +899,12 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
       if (tid == 0) {
         es->nlive = nlive + ktot;
         es->npend = 2 * ktot;
+        es->ref = 0;
       }
       } while (0);
       engine_cluster_sync<CS>();
       if (es0->stop) break;
+      if (!REF || !es0->ref) ++sweep;
     }
     if (crank == 0) pol.end_job(job, es->V, es->E, es->neval, es->status);
     __syncthreads();

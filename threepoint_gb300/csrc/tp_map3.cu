@@ -57,19 +57,29 @@ struct Map3Policy {
     float lo;  // log2(l1 l2 uHat uHat uHat)
     int live;
   };
+  // FP64: the integer-arithmetic triangle (27 64-bit words, odd again), or
+  // (tri.ok = 0) the triangle of the FP64 instructions; live when outer != 0
   struct RecD {
-    Tri<double> tri;
+    union {
+      Tri64 tri;
+      Tri<double> f64;
+    };
     double outer;  // l1 l2 uHat uHat uHat
-    int live;
   };
   typedef typename std::conditional<sizeof(R) == 4, RecF, RecD>::type Rec;
   const int* job_order;
+  static constexpr bool REF = sizeof(R) == 8;  // FP64 instructions beside the integer form
+  int ref = 0;
   static constexpr int REC = (int)sizeof(Rec);
   static constexpr int PD = 1;
   static constexpr int NS = 1;
   __device__ static int slot(int) { return 0; }
   static constexpr size_t PLT_BYTES = (sizeof(R) == 4 && !TP_MAP3_PLT_GLOBAL) ? sizeof(float4) * PLT_N : 0;
-  static constexpr size_t PSMEM = sizeof(R) * NCP * NNODE + sizeof(CosmoK<R>) + sizeof(BulkBar) + 128 + PLT_BYTES;
+  // node table of the job's cosmology in shared memory: NF_* rows or Node64
+  static constexpr size_t NODE_BYTES = sizeof(R) == 4 ? sizeof(R) * NCP * NNODE : sizeof(Node64) * NNODE;
+  static constexpr size_t EX2_BYTES = sizeof(R) == 4 ? 0 : sizeof(I64Tables::ex2);
+  static constexpr size_t PSMEM =
+      NODE_BYTES + EX2_BYTES + sizeof(CosmoK<R>) + sizeof(BulkBar) + 128 + PLT_BYTES;
 
   // inputs
   const int* job_cosmo;
@@ -94,7 +104,7 @@ struct Map3Policy {
   double scale;
 
   __device__ BulkBar* bar(char* psmem) {
-    return (BulkBar*)(psmem + sizeof(R) * NCP * NNODE + ((sizeof(CosmoK<R>) + 15) & ~size_t(15)));
+    return (BulkBar*)(psmem + NODE_BYTES + EX2_BYTES + ((sizeof(CosmoK<R>) + 15) & ~size_t(15)));
   }
   __device__ unsigned long long* live_counter(char* psmem) {
     return (unsigned long long*)((char*)bar(psmem) + ((sizeof(BulkBar) + 15) & ~size_t(15)));
@@ -104,19 +114,27 @@ struct Map3Policy {
 
   __device__ void begin_job(int job, char* psmem, double* xmin, double* xmax) {
     s_nc = (R*)psmem;
-    s_ck = (CosmoK<R>*)(psmem + sizeof(R) * NCP * NNODE);
+    s_ck = (CosmoK<R>*)(psmem + NODE_BYTES + EX2_BYTES);
     const int c = job_cosmo[job];
     if (c != cur_cosmo) {
       __syncthreads();
-      const R* src = node_coef + (size_t)c * NCP * NNODE;
-      constexpr int nbytes = (int)(sizeof(R) * NCP * NNODE);
+      const char* src;
+      if constexpr (sizeof(R) == 4)
+        src = (const char*)(node_coef + (size_t)c * NCP * NNODE);
+      else
+        src = (const char*)ck[c].n64;
+      constexpr int nbytes = (int)NODE_BYTES;
       static_assert(nbytes % 16 == 0, "bulk copy size must be a multiple of 16 bytes");
       if (threadIdx.x == 0) {
         // the node table (10-20 KB) is staged by one bulk async copy
-        if (!bulk_copy_g2s(bar(psmem), s_nc, src, nbytes)) {
-          for (int i = 0; i < NCP * NNODE; ++i) s_nc[i] = src[i];
+        if (!bulk_copy_g2s(bar(psmem), psmem, src, nbytes)) {
+          for (int i = 0; i < nbytes / 4; ++i) ((uint32_t*)psmem)[i] = ((const uint32_t*)src)[i];
         }
         *s_ck = ck[c];
+      }
+      if constexpr (sizeof(R) == 8) {
+        uint64_t* ex = (uint64_t*)(psmem + NODE_BYTES);
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) ex[i] = d_i64tab.ex2[i];
       }
       __syncthreads();
       if constexpr (sizeof(R) == 4 && !TP_MAP3_PLT_GLOBAL) {
@@ -152,6 +170,20 @@ struct Map3Policy {
     __syncthreads();
   }
 
+  // the reference form's point; a function of its own, so that what the
+  // compiler contracts in it does not depend on the fast form around it
+  static __device__ __noinline__ bool setup_f64(const double* x, const double* th, RecD& r) {
+    double l1 = x[0], l2 = x[1], phi = x[2];
+    double s = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(phi);
+    double l3 = s > 0 ? sqrt(s) : 0.0;
+    double outer = l1 * l2 * uhat(l1 * th[0]) * uhat(l2 * th[1]) * uhat(l3 * th[2]);
+    bool live = !(l1 == 0 || l2 == 0 || l3 == 0) && l1 > 1.0e-10 && l2 > 1.0e-10 && l3 > 1.0e-10 && outer != 0.0;
+    r.outer = live ? outer : 0.0;
+    r.tri.ok = 0;
+    if (live) make_tri<double>(l1, l2, l3, r.f64);
+    return live;
+  }
+
   // returns whether the point needs its line-of-sight sum
   __device__ bool setup(int p, const double* x, char* recp) {
     (void)p;
@@ -183,16 +215,17 @@ struct Map3Policy {
         trif_from_tri(t, r.tri);
       }
     } else {
+      if (ref || !s_ck->c64.ok) return setup_f64(x, th, r);
       double l1 = x[0], l2 = x[1], phi = x[2];
       double s = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(phi);
       double l3 = s > 0 ? sqrt(s) : 0.0;
       double outer = l1 * l2 * uhat(l1 * th[0]) * uhat(l2 * th[1]) * uhat(l3 * th[2]);
       live = !(l1 == 0 || l2 == 0 || l3 == 0) && l1 > 1.0e-10 && l2 > 1.0e-10 && l3 > 1.0e-10 && outer != 0.0;
-      r.outer = outer;
-      if (live) make_tri<R>(l1, l2, l3, r.tri);
+      r.outer = live ? outer : 0.0;
+      if (live && !tri64_record(l1, l2, l3, *s_ck, r.tri)) setup_f64(x, th, r);
     }
-    r.live = live;
-    if (live && nlive) atomicAdd(s_live, 1ull);
+    if constexpr (sizeof(R) == 4) r.live = live;
+    if (live && nlive && !ref) atomicAdd(s_live, 1ull);
     return live;
   }
 
@@ -237,22 +270,20 @@ struct Map3Policy {
       }
       pv[0] = (double)(s.x + s.y);  // lanes added in FP32: one conversion, no FP64 add per item
     } else {
-      KSum<R> acc;
-      TP_UNROLL(TP_MAP3_UNROLL)
-      for (int j = j0; j < j0 + NPG; ++j) {
-        R v = bispec_node<R>(s_nc, j, r.tri, K);
-        if (v != v) v = (R)0;  // NaN in bispec -> 0 (bispectrum.cu:327-331)
-        acc.add(v);
-      }
-      pv[0] = (double)acc.s;
+      const R* nc = node_coef + (size_t)cur_cosmo * NCP * NNODE;
+      pv[0] = r.tri.ok ? bkappa64_nodes((const Node64*)s_nc, nc, j0, NPG, r.tri, K,
+                                        (const uint64_t*)((const char*)s_nc + NODE_BYTES))
+                       : bkappa_nodes_f64(nc, j0, NPG, r.f64, K);
     }
   }
 
-  __device__ bool is_live(const char* recp) const { return ((const Rec*)recp)->live != 0; }
+  __device__ static bool rec_live(const RecF& r) { return r.live != 0; }
+  __device__ static bool rec_live(const RecD& r) { return r.outer != 0.0; }
+  __device__ bool is_live(const char* recp) const { return rec_live(*(const Rec*)recp); }
 
   __device__ void finalize(const char* recp, const double* sum, double* fv) {
     const Rec& r = *(const Rec*)recp;
-    if (!r.live) {
+    if (!rec_live(r)) {
       fv[0] = 0.0;
       return;
     }
@@ -288,7 +319,7 @@ struct Map3Policy {
 // CS > 1: one cluster of CS CTAs per integral (the cooperative form of
 // adaptive_body), for batches with fewer integrals than CTA slots
 template <typename R, int NT, int CS>
-__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? TP_MAP3_MINB : 1) k_map3(Map3Policy<R> pol_in, int njobs, int* job_counter, EngineCfg cfg,
+__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? TP_MAP3_MINB : 2) k_map3(Map3Policy<R> pol_in, int njobs, int* job_counter, EngineCfg cfg,
                                              char* scratch, size_t slot_bytes) {
   Map3Policy<R> pol = pol_in;
   pol.cur_cosmo = -1;
@@ -313,11 +344,10 @@ size_t map3_smem_bytes() {
 }
 
 // ---------------------------------------------------------------------------
-// Point evaluation of b_kappa (no cubature): one warp per point, 3 nodes per
-// lane, shuffle reduction.
-template <typename R>
-__global__ void k_bkappa_points(const int* cosmo_idx, const double* ell, long n, const R* node_coef,
-                                const double* wscale, const CosmoK<R>* ck, double* out) {
+// Point evaluation of b_kappa (no cubature), FP32: one warp per point, 3 nodes
+// per lane, shuffle reduction.
+__global__ void k_bkappa_points_f32(const int* cosmo_idx, const double* ell, long n, const float* node_coef,
+                                    const double* wscale, const CosmoK<float>* ck, double* out) {
   long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
   if (w >= n) return;
@@ -327,29 +357,67 @@ __global__ void k_bkappa_points(const int* cosmo_idx, const double* ell, long n,
     if (lane == 0) out[w] = 0.0;
     return;
   }
-  Tri<R> T;
-  make_tri<R>(l1, l2, l3, T);
-  const R* nc = node_coef + (size_t)c * NCP * NNODE;
-  const CosmoK<R> K = ck[c];
-  KSum<R> acc;
-  if constexpr (sizeof(R) == 4) {
-    TriF F;
-    trif_from_tri(T, F);
-    for (int j = lane; j < NNODE; j += 32) {
-      float v = bispec_node_fast(nc, j, F, K);
-      if (v != v) v = 0.f;
-      acc.add(v);
-    }
-  } else {
-    for (int j = lane; j < NNODE; j += 32) {
-      R v = bispec_node<R>(nc, j, T, K);
-      if (v != v) v = (R)0;
-      acc.add(v);
-    }
+  Tri<float> T;
+  make_tri<float>(l1, l2, l3, T);
+  const float* nc = node_coef + (size_t)c * NCP * NNODE;
+  const CosmoK<float> K = ck[c];
+  KSum<float> acc;
+  TriF F;
+  trif_from_tri(T, F);
+  for (int j = lane; j < NNODE; j += 32) {
+    float v = bispec_node_fast(nc, j, F, K);
+    if (v != v) v = 0.f;
+    acc.add(v);
   }
   double s = (double)acc.s;
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) out[w] = s * wscale[c];
+}
+
+// FP64: a block takes BK_PTS points; one thread a point sets its triangle up
+// in shared memory, then every thread sums the nodes of one (point, node
+// group) item, a warp's lanes at one group of neighbouring points, so that a
+// node row is one broadcast load.
+constexpr int BK_PTS = 32, BK_G = 8;
+__global__ void __launch_bounds__(BK_PTS* BK_G, 2)
+    k_bkappa_points_f64(const int* cosmo_idx, const double* ell, long n, const double* node_coef,
+                        const double* wscale, const CosmoK<double>* ck, double* out) {
+  __shared__ Tri64 tri[BK_PTS];
+  __shared__ uint64_t ex2[256];
+  __shared__ double part[BK_G][BK_PTS];
+  static_assert(BK_PTS * BK_G == 256, "the table load takes one entry a thread");
+  const int q = threadIdx.x % BK_PTS, g = threadIdx.x / BK_PTS;
+  const long p = (long)blockIdx.x * BK_PTS + q;
+  ex2[threadIdx.x] = d_i64tab.ex2[threadIdx.x];
+  bool live = p < n;
+  int c = 0;
+  if (live) {
+    c = cosmo_idx ? cosmo_idx[p] : 0;
+    const double l1 = ell[3 * p], l2 = ell[3 * p + 1], l3 = ell[3 * p + 2];
+    live = l1 > 1e-10 && l2 > 1e-10 && l3 > 1e-10;
+    if (g == 0 && live) tri64_record(l1, l2, l3, ck[c], tri[q]);
+  }
+  __syncthreads();
+  double v = 0.0;
+  if (live) {
+    const CosmoK<double>& K = ck[c];
+    const double* nc = node_coef + (size_t)c * NCP * NNODE;
+    if (tri[q].ok) {
+      v = bkappa64_nodes(K.n64, nc, g * (NNODE / BK_G), NNODE / BK_G, tri[q], K, ex2);
+    } else {
+      Tri<double> T;
+      make_tri<double>(ell[3 * p], ell[3 * p + 1], ell[3 * p + 2], T);
+      v = bkappa_nodes_f64(nc, g * (NNODE / BK_G), NNODE / BK_G, T, K);
+    }
+  }
+  part[g][q] = v;
+  __syncthreads();
+  if (g == 0 && p < n) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < BK_G; ++k) s += part[k][q];
+    out[p] = live ? s * wscale[c] : 0.0;
+  }
 }
 
 // Per-node terms of b_kappa at given triangles (no cubature), with the
@@ -403,7 +471,12 @@ __global__ void k_bkappa_nodes(int c, const double* ell, long n, const R* node_c
     }
   } else {
     const R* row = nc + (size_t)u * NCP;
-    const R B = bispec_eval<R>(row, 1, row[NC_S], row[NC_L2S], row[NC_HF], row[NC_L2HF], T, K);
+    Tri64 T6;
+    R B;
+    if (K.c64.ok && K.n64[u].ok && tri64_record(l1, l2, l3, K, T6))
+      B = bispec64(K.n64[u], T6, K.c64, d_i64tab.ex2);
+    else
+      B = bispec_eval<R>(row, 1, row[NC_S], row[NC_L2S], row[NC_HF], row[NC_L2HF], T, K);
     R v = row[NC_W] * B;
     if (v != v) v = (R)0;
     term[i * NNODE + u] = (double)v * wscale[c];
@@ -428,7 +501,7 @@ cudaError_t launch_bkappa_nodes(int precision, int cosmo, const double* ell, lon
 // ---------------------------------------------------------------------------
 constexpr int MAP3_NT = 256;
 
-constexpr int MAP3_CLUSTER = 8;
+constexpr int MAP3_CLUSTER = 8, MAP3_CLUSTER_MAX = 16;
 
 static cudaLaunchConfig_t map3_launch_config(int grid, size_t smem, cudaStream_t st, int cluster,
                                              cudaLaunchAttribute* attr) {
@@ -446,10 +519,28 @@ static cudaLaunchConfig_t map3_launch_config(int grid, size_t smem, cudaStream_t
   return lc;
 }
 
-// grid of CTAs (a multiple of *cluster), one CTA per integral, or one
-// MAP3_CLUSTER-CTA cluster per integral (*cluster = MAP3_CLUSTER) when
-// allow_cluster is 1 and the batch has no more integrals than CTA slots, or
-// allow_cluster is 2;
+// clusters of CS CTAs that the device holds at once (0: they do not fit)
+template <typename R, int CS>
+static int map3_clusters(size_t smem) {
+  int n = 0;
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t lc = map3_launch_config(CS, smem, 0, CS, attr);
+  auto kern = k_map3<R, MAP3_NT, CS>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // clusters of more than 8 CTAs are a non-portable size (allowed on GB300)
+  if (e == cudaSuccess && CS > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &lc);
+  cudaGetLastError();
+  return e == cudaSuccess ? n : 0;
+}
+
+// grid of CTAs (a multiple of *cluster), one CTA per integral, or one cluster
+// of *cluster CTAs per integral when allow_cluster is 1 and the batch leaves
+// CTA slots idle otherwise (16 CTAs where that many per integral fit the
+// slots at once, else 8 where the batch has no more integrals than slots: ten
+// FP64 integrals take 93 ms on 16-CTA clusters and 130 ms on 8-CTA ones with
+// the table build, twenty FP32 ones 33.6 and 35.9 ms), or
+// 8 CTAs for every batch when allow_cluster is 2;
 // *scratch = bytes of the region stores (one per CTA or per cluster)
 template <typename R>
 static cudaError_t plan_map3_t(int njobs, int cap, int max_ctas, int allow_cluster, int* grid, int* cluster,
@@ -467,23 +558,19 @@ static cudaError_t plan_map3_t(int njobs, int cap, int max_ctas, int allow_clust
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   int g = sms * per_sm;
   if (max_ctas > 0 && g > max_ctas) g = max_ctas;
-  if ((allow_cluster == 2 || (allow_cluster == 1 && njobs <= g)) && (max_ctas <= 0 || max_ctas >= MAP3_CLUSTER)) {
-    int nclusters = 0;
-    cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t lc = map3_launch_config(MAP3_CLUSTER, *smem, 0, MAP3_CLUSTER, attr);
-    e = cudaFuncSetAttribute(k_map3<R, MAP3_NT, MAP3_CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)*smem);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveClusters(&nclusters, (const void*)k_map3<R, MAP3_NT, MAP3_CLUSTER>, &lc);
-    cudaGetLastError();
-    if (e == cudaSuccess && nclusters >= 1) {
-      if (max_ctas > 0) nclusters = std::min(nclusters, max_ctas / MAP3_CLUSTER);
-      nclusters = std::min(nclusters, njobs);
-      *cluster = MAP3_CLUSTER;
-      *grid = nclusters * MAP3_CLUSTER;
-      *scratch = (size_t)nclusters * Slot<3, 1>::bytes(cap);
-      return cudaSuccess;
-    }
+  for (int cs : {MAP3_CLUSTER_MAX, MAP3_CLUSTER}) {
+    const bool want = allow_cluster == 2 ? cs == MAP3_CLUSTER
+                                         : allow_cluster == 1 && (cs == MAP3_CLUSTER ? njobs <= g : (long)njobs * cs <= g);
+    if (!want || (max_ctas > 0 && max_ctas < cs)) continue;
+    int nclusters = cs == MAP3_CLUSTER ? map3_clusters<R, MAP3_CLUSTER>(*smem) : map3_clusters<R, MAP3_CLUSTER_MAX>(*smem);
+    if (max_ctas > 0) nclusters = std::min(nclusters, max_ctas / cs);
+    if (cs == MAP3_CLUSTER_MAX && nclusters < njobs) continue;  // 8-CTA clusters hold them all at once
+    if (nclusters < 1) continue;
+    nclusters = std::min(nclusters, njobs);
+    *cluster = cs;
+    *grid = nclusters * cs;
+    *scratch = (size_t)nclusters * Slot<3, 1>::bytes(cap);
+    return cudaSuccess;
   }
   if (g > njobs) g = njobs;
   if (g < 1) g = 1;
@@ -535,10 +622,12 @@ static cudaError_t launch_map3_t(const Map3Launch& L, int grid, size_t smem, cha
   pol.job_order = L.job_order;
   EngineCfg cfg{0.0, L.rel_tol, TP_NORM_L1, L.cap, L.max_sweeps};
   size_t slot = Slot<3, 1>::bytes(L.cap);
-  if (L.cluster == MAP3_CLUSTER) {
+  if (L.cluster > 1) {
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t lc = map3_launch_config(grid, smem, st, MAP3_CLUSTER, attr);
-    return cudaLaunchKernelEx(&lc, k_map3<R, MAP3_NT, MAP3_CLUSTER>, pol, L.njobs, L.job_counter, cfg, scratch, slot);
+    cudaLaunchConfig_t lc = map3_launch_config(grid, smem, st, L.cluster, attr);
+    return L.cluster == MAP3_CLUSTER
+               ? cudaLaunchKernelEx(&lc, k_map3<R, MAP3_NT, MAP3_CLUSTER>, pol, L.njobs, L.job_counter, cfg, scratch, slot)
+               : cudaLaunchKernelEx(&lc, k_map3<R, MAP3_NT, MAP3_CLUSTER_MAX>, pol, L.njobs, L.job_counter, cfg, scratch, slot);
   }
   k_map3<R, MAP3_NT, 1><<<grid, MAP3_NT, smem, st>>>(pol, L.njobs, L.job_counter, cfg, scratch, slot);
   return cudaGetLastError();
@@ -551,15 +640,13 @@ cudaError_t launch_map3(const Map3Launch& L, int grid, size_t smem, char* scratc
 
 cudaError_t launch_bkappa_points(int precision, const int* cosmo_idx, const double* ell, long n, const void* ncoef,
                                  const double* wscale, const void* ck, double* out, cudaStream_t st) {
-  long threads = n * 32;
-  int bs = 256;
-  unsigned grid = (unsigned)((threads + bs - 1) / bs);
+  const int bs = 256;
   if (precision == TP_FP64)
-    k_bkappa_points<double><<<grid, bs, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
-                                                  (const CosmoK<double>*)ck, out);
+    k_bkappa_points_f64<<<(unsigned)((n + BK_PTS - 1) / BK_PTS), BK_PTS * BK_G, 0, st>>>(
+        cosmo_idx, ell, n, (const double*)ncoef, wscale, (const CosmoK<double>*)ck, out);
   else
-    k_bkappa_points<float><<<grid, bs, 0, st>>>(cosmo_idx, ell, n, (const float*)ncoef, wscale,
-                                                 (const CosmoK<float>*)ck, out);
+    k_bkappa_points_f32<<<(unsigned)((n * 32 + bs - 1) / bs), bs, 0, st>>>(
+        cosmo_idx, ell, n, (const float*)ncoef, wscale, (const CosmoK<float>*)ck, out);
   return cudaGetLastError();
 }
 

@@ -740,6 +740,57 @@ TP_TABLE_KERNEL k_plin_table(const CosmoDev* cos, const EHConst* eh, float4* plt
   if (a == 0 && threadIdx.x == 0 && !c.pk_given) ck32[ci].plt = (const float*)(plt + (size_t)ci * PLT_N);
 }
 
+// P_lin table of the integer-arithmetic integrands (P64Cell), one thread per cell
+TP_TABLE_KERNEL k_p64(const CosmoDev* cos, const EHConst* eh, P64Cell* p64, CosmoK<double>* ck64, int n) {
+  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int ci = (int)(idx / P64_N), i = (int)(idx % P64_N);
+  if (ci >= n || cos[ci].pk_given) return;
+  const EHConst& e = eh[ci];
+  P64Cell c;
+  if (p64_cell(i, e.omh2, e.sa, e.one_m_sa, 0.43 * e.sh, e.theta2, e.c184, e.ehc, e.ns, d_i64tab, c))
+    p64[idx] = c;
+  else
+    ck64[ci].c64.bad = 1;
+}
+
+// node rows of the integer-arithmetic integrands from the NC_* rows; the
+// cosmology takes that form when its P(k) is the fit's, its constants are
+// ordinary numbers and some ell range keeps every node inside the P table
+TP_TABLE_KERNEL k_node64(const CosmoDev* cos, const EHConst* eh, const double* ncoef, const P64Cell* p64, Node64* n64,
+                         CosmoK<double>* ck64, int n) {
+  const int ci = blockIdx.x;
+  if (ci >= n) return;
+  double lo = 0x1p-36, hi = 0x1p26;
+  for (int j = threadIdx.x; j < NNODE; j += 32) {
+    const double* v = ncoef + ((size_t)ci * NNODE + j) * NCP;
+    Node64& N = n64[(size_t)ci * NNODE + j];
+    node64_make(v[NC_W], v[NC_S], v[NC_HF], v[NC_ANA], v[NC_ANR], v[NC_ANC], v[NC_BN], v[NC_CN], v[NC_ALA], v[NC_ALD],
+                v[NC_BETAB], v[NC_FN], v[NC_GN], v[NC_HN], v[NC_MN], v[NC_NN], v[NC_MUN], v[NC_NUN], v[NC_PN],
+                v[NC_EN], v[NC_DN], v[NC_D1SQ], v[NC_TREE] != 0.0, d_i64tab, N);
+    if (N.ok) {
+      lo = fmax(lo, exp2(P64_LO + 0.01 - v[NC_L2HF]));
+      hi = fmin(hi, exp2(P64_HI - 0.01 - v[NC_L2HF]));
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmax(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmin(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (threadIdx.x == 0) {
+    const EHConst& e = eh[ci];
+    const double amax = 1. - (2. / 3.) * cos[ci].ns;
+    CosmoK<double>& k = ck64[ci];
+    k.n64 = n64 + (size_t)ci * NNODE;
+    k.c64.p = p64 + (size_t)ci * P64_N;
+    k.c64.ok = !k.c64.bad && !cos[ci].pk_given && amax >= 0 && fabs(e.ns) < 3 && sf_ok(e.ehc) && sf_ok(e.omh2) && sf_ok(e.sa) &&
+               e.one_m_sa > -0.5 * e.sa && sf_ok(e.theta2) && e.c184 > 1e-6 && e.c184 < 1e6 && e.sh > 1e-3 &&
+               e.sh < 1e6 && e.omh2 > 1e-6 && e.omh2 < 1e6 && lo < hi;
+    k.c64.amax = k.c64.ok ? (uint64_t)i64_fix<59>(amax) : 0;
+    k.c64.lo = lo;
+    k.c64.hi = hi;
+  }
+}
+
 // ---------------------------------------------------------------------------
 void upload_gauss_nodes() {
   double a[48], w[48];
@@ -752,7 +803,7 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
                          double* d_ncoef, float* d_ncoef_f, float* d_fcoef_f, double* d_hcoef, float* d_hcoef_f,
                          double* d_wscale64,
                          double* d_wscale32, CosmoK<double>* d_ck64, CosmoK<float>* d_ck32, float4* d_plt,
-                         double* d_ehg, int n, cudaStream_t s) {
+                         double* d_ehg, Node64* d_n64, P64Cell* d_p64, int n, cudaStream_t s) {
   // every launch is made of one-warp blocks (see above). An SM runs blocks of
   // different kernels together only in one shared-memory/L1 configuration:
   // these kernels ask for the one k_map3 runs in (maximum shared memory).
@@ -778,7 +829,7 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
     cudaGetLastError();  // a failed query leaves rsigma_smem = 0
     const void* ks[] = {(const void*)k_eh_table, (const void*)k_norm, (const void*)k_fk, (const void*)k_g, (const void*)k_growth,
                         (const void*)k_rsigma, (const void*)k_node_coefs, (const void*)k_finish,
-                        (const void*)k_plin_table};
+                        (const void*)k_plin_table, (const void*)k_p64, (const void*)k_node64};
     for (const void* k : ks)
       cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     carveout_set = dev;
@@ -793,6 +844,8 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
   k_finish<<<n, 32, 0, s>>>(d_cos, d_eh, d_tab, d_ncoef, d_ncoef_f, d_fcoef_f, d_wscale64, d_wscale32, d_ck64, d_ck32,
                             n);
   k_plin_table<<<n * (PLT_N / 128), 32, 0, s>>>(d_cos, d_eh, d_plt, d_ck32, n);
+  k_p64<<<(unsigned)((long)n * P64_N / 32), 32, 0, s>>>(d_cos, d_eh, d_p64, d_ck64, n);
+  k_node64<<<n, 32, 0, s>>>(d_cos, d_eh, d_ncoef, d_p64, d_n64, d_ck64, n);
   return cudaGetLastError();
 }
 
