@@ -185,7 +185,8 @@ __device__ inline void rule_axis(const double* f, int* split, bool* split_tie) {
 #pragma unroll
     for (int d = 0; d < DIM; ++d) {
       double v0 = V(1 + 4 * d), v1 = V(2 + 4 * d), v2 = V(3 + 4 * d), v3 = V(4 + 4 * d);
-      diff[d] += fabs(v0 + v1 - 2 * val0 - GM::ratio * (v2 + v3 - 2 * val0));
+      const double da = __dsub_rn(__dadd_rn(v0, v1), 2 * val0), db = __dsub_rn(__dadd_rn(v2, v3), 2 * val0);
+      diff[d] += fabs(fma(-GM::ratio, db, da));
     }
   }
   double md = 0;
@@ -275,16 +276,21 @@ __device__ inline void rule_combine(const double* f, double vol, double hw0, dou
         double v0 = V(1 + 4 * d), v1 = V(2 + 4 * d), v2 = V(3 + 4 * d), v3 = V(4 + 4 * d);
         s2 += v0 + v1;
         s3 += v2 + v3;
-        diff[d] += fabs(v0 + v1 - 2 * val0 - GM::ratio * (v2 + v3 - 2 * val0));
+        const double da = __dsub_rn(__dadd_rn(v0, v1), 2 * val0), db = __dsub_rn(__dadd_rn(v2, v3), 2 * val0);
+        diff[d] += fabs(fma(-GM::ratio, db, da));
       }
       int k0 = 1 + 4 * DIM;
       for (int i = 0; i < 2 * DIM * (DIM - 1); ++i) s4 += V(k0 + i);
       k0 += 2 * DIM * (DIM - 1);
       for (int i = 0; i < (1 << DIM); ++i) s5 += V(k0 + i);
-      double r7 = vol * (w1 * val0 + w2 * s2 + w3 * s3 + w4 * s4 + w5 * s5);
-      double r5 = vol * (wE1 * val0 + wE2 * s2 + wE3 * s3 + wE4 * s4);
+      // explicit roundings: what the compiler contracts here would depend on the
+      // code around the inlined rule, and bitwise ties of errors decide splits
+      const double x7 = fma(w5, s5, fma(w4, s4, fma(w3, s3, fma(w2, s2, __dmul_rn(w1, val0)))));
+      const double x5 = fma(wE4, s4, fma(wE3, s3, fma(wE2, s2, __dmul_rn(wE1, val0))));
+      const double r7 = __dmul_rn(vol, x7);
+      const double dr = fma(vol, x5, -r7);
       val[k] = r7;
-      err[k] = fabs(r5 - r7);
+      err[k] = fabs(dr);
     }
     double md = 0;
     int dm = 0;
@@ -328,31 +334,6 @@ __device__ inline double block_sum(double v, double* red) {
   return t;
 }
 
-template <int NT>
-__device__ inline int block_exclusive_scan(int v, int* red, int* total) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  int x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (l >= o) x += y;
-  }
-  __syncthreads();
-  if (l == 31) red[w] = x;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int t = (l < NT / 32) ? red[l] : 0;
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, t, o);
-      if (l >= o) t += y;
-    }
-    red[l + 32] = t;  // inclusive warp-prefix of warp totals
-  }
-  __syncthreads();
-  int base = (w > 0) ? red[32 + w - 1] : 0;
-  *total = red[32 + NT / 32 - 1];
-  return base + x - v;
-}
-
 __device__ inline bool converged_check(int fdim, int norm, const double* V, const double* E, double abs_tol,
                                        double rel_tol) {
   if (fdim == 1 || norm == TP_NORM_INDIVIDUAL) {
@@ -372,14 +353,15 @@ __device__ inline bool converged_check(int fdim, int norm, const double* V, cons
 // Shared scratch of the engine (besides the policy's own)
 template <int FDIM>
 struct EngineShared {
-  int live_list[1024];  // live points of the current chunk
+  int live_list[1024];  // live points of the current chunk; the selection's last candidates
   int nlive_chunk;
   unsigned long long hist[256];
   double red[64];
   int ired[80];
   double V[FDIM], E[FDIM];
   unsigned long long q_above;
-  unsigned long long prefix;
+  unsigned long long prefix, qtot;
+  int digit;
   int job, nlive, npend, status, stop, ktot, sweeps, ref, nband, nref, nfull;
   long long neval;
 };
@@ -392,6 +374,362 @@ __host__ __device__ constexpr size_t engine_smem_bytes() {
          sizeof(double) * (size_t)P::CH * GMRule<DIM>::NP * FDIM + sizeof(EngineShared<FDIM>) + 16;
 }
 
+
+// ---------------------------------------------------------------------------
+// One sweep's bookkeeping by the NT threads of one CTA: the totals, the
+// convergence test, the choice of the regions to split (every region whose
+// error is at least the largest tau that leaves a remaining error within the
+// tolerance), and their splitting into S.pend. Sets es->stop, or es->npend,
+// es->nlive, es->ref.
+//
+// The other CTAs of a cluster wait for it, and it is a chain of passes over
+// the region store with barriers between them, so its latency counts: the
+// error keys are read once and staged in shared memory (stage: the point
+// records and partial sums, idle between evaluations) for the radix passes,
+// regions above the last 32 candidates are settled by one warp, and the
+// chosen regions are split one per thread from a list. Measured with the
+// earlier form (keys read again from the region store in each of eight passes,
+// a contiguous range of regions split by each thread): a <Map^3> integral's
+// sweep of ~1500 regions 60k -> 33k cycles, a Gamma one of ~3000 160k -> 60k;
+// 64 FP32 Gamma triangles with the set-up of GammaPolicy 340 -> 240 ms.
+template <int DIM, int FDIM, int NT, bool REF>
+__device__ __forceinline__ void engine_select(Slot<DIM, FDIM> S, EngineShared<FDIM>* es, EngineCfg cfg,
+                                              unsigned long long* stage, int stage_bytes, int sweep, int npend,
+                                              int ref) {
+  constexpr int NP = GMRule<DIM>::NP;
+  typedef unsigned long long u64;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0 && !ref) es->neval += (long long)npend * NP;
+
+  // ---------------- totals and convergence ----------------------------
+  const int nlive = es->nlive;
+  // staged: the key and, with several components, the error sum
+  constexpr int SW = FDIM == 1 ? 1 : 2;
+  const int nst = min(nlive, stage_bytes / (8 * SW));
+  double tv[FDIM], te[FDIM];
+#pragma unroll
+  for (int k = 0; k < FDIM; ++k) tv[k] = te[k] = 0;
+#pragma unroll 4
+  for (int i = tid; i < nlive; i += NT) {
+    double ev[FDIM];
+#pragma unroll
+    for (int k = 0; k < FDIM; ++k) {
+      tv[k] += S.val[(size_t)k * S.cap + i];
+      ev[k] = S.err[(size_t)k * S.cap + i];
+      te[k] += ev[k];
+    }
+    if (i < nst) {
+      stage[i] = (u64)__double_as_longlong(S.emax[i]);
+      if constexpr (SW == 2) {
+        double es_ = 0;
+#pragma unroll
+        for (int k = 0; k < FDIM; ++k) es_ += ev[k];
+        stage[nst + i] = (u64)__double_as_longlong(es_);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < FDIM; ++k) {
+    tv[k] = block_sum<NT>(tv[k], es->red);
+    te[k] = block_sum<NT>(te[k], es->red);
+  }
+  auto finish = [&](int bits) {
+    if (tid == 0) {
+      for (int k = 0; k < FDIM; ++k) {
+        es->V[k] = tv[k];
+        es->E[k] = te[k];
+      }
+      es->status |= bits;
+      es->sweeps = sweep + 1;
+      es->stop = 1;
+    }
+    __syncthreads();
+  };
+  const bool conv = converged_check(FDIM, cfg.norm, tv, te, cfg.abs_tol, cfg.rel_tol);
+  if (conv || sweep + 1 >= cfg.max_sweeps) return finish(conv ? 0 : 2);
+  // tolerance for the Gladwell pop loop
+  double etot = 0, vabs = 0;
+  bool l1 = !(FDIM == 1 || cfg.norm == TP_NORM_INDIVIDUAL);
+#pragma unroll
+  for (int k = 0; k < FDIM; ++k) {
+    etot += te[k];
+    vabs += fabs(tv[k]);
+  }
+  const double tol = fmax(cfg.abs_tol, (l1 ? vabs : fabs(tv[0])) * cfg.rel_tol);
+
+  // ---------------- radix select of the error threshold ---------------
+  // Errors are summed as 62-bit fixed-point fractions of the total error,
+  // so the histogram sums (shared-memory integer atomics) are exact and
+  // independent of the order of the additions.
+  const double qscale = 4.611686018427387904e18 / etot;  // 2^62 / E_tot
+  const double tol_q = tol * qscale;
+  auto key_of = [&](int i) { return i < nst ? stage[i] : (u64)__double_as_longlong(S.emax[i]); };
+  auto q_of = [&](int i, u64 key) {
+    double es_;
+    if constexpr (FDIM == 1) {
+      es_ = __longlong_as_double((long long)key);
+    } else if (i < nst) {
+      es_ = __longlong_as_double((long long)stage[nst + i]);
+    } else {
+      es_ = 0;
+#pragma unroll
+      for (int k = 0; k < FDIM; ++k) es_ += S.err[(size_t)k * S.cap + i];
+    }
+    return (u64)(es_ * qscale);
+  };
+  // Digits of the keys, largest first: the first pass takes 255 bins of 1/8
+  // octave below the largest key (one byte of the exponent would put all
+  // regions into two or three bins, whose shared-memory atomics then queue:
+  // 20 us a sweep); a cut below those, and the rest of the key, go by bytes.
+  // Keys whose first bits (key >> sh) equal pre are the candidates; they are
+  // listed once they fit.
+  constexpr int LIST = 1024;
+  int hmax = 0;
+  for (int i = tid; i < nlive; i += NT) hmax = max(hmax, (int)(key_of(i) >> 32));
+  hmax = __reduce_max_sync(0xffffffffu, hmax);
+  if (lane == 0) es->ired[warp] = hmax;
+  if (tid == 0) {
+    es->prefix = 0ull;
+    es->q_above = 0ull;
+  }
+  __syncthreads();
+  for (int w = 0; w < NT / 32; ++w) hmax = max(hmax, es->ired[w]);
+  const int top = hmax >> 17;  // of key >> 49
+  int ncand = -1, sh = 64;
+  u64 pre = 0, qtot = 0, tau = 0;
+  for (bool octaves = true;; octaves = false) {
+    const int w = min(8, sh), nsh = octaves ? 49 : sh - w;
+    for (int b = tid; b < 256; b += NT) es->hist[b] = 0ull;
+    if (tid == 0) es->nlive_chunk = 0;
+    __syncthreads();
+    auto count = [&](int i) {
+      const u64 key = key_of(i);
+      if (octaves) {
+        atomicAdd(&es->hist[max(0, 255 - (top - (int)(key >> 49)))], q_of(i, key));
+      } else if (sh == 64 || (key >> sh) == pre) {
+        atomicAdd(&es->hist[(key >> nsh) & ((1u << w) - 1)], q_of(i, key));
+      }
+    };
+    if (ncand >= 0) {
+      for (int c = tid; c < ncand; c += NT) count(es->live_list[c]);
+    } else {
+      for (int i = tid; i < nlive; i += NT) count(i);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      const int l = tid;
+      u64 loc[8];
+      u64 ls = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        loc[q] = es->hist[8 * l + q];
+        ls += loc[q];
+      }
+      u64 all = ls;
+      for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+      // the first pass histograms every region: its sum is the fixed-point total
+      const u64 qt = octaves ? all : es->qtot;
+      // suffix sum over lanes (lane l: sum of lanes > l)
+      u64 suf = ls;
+      for (int o = 1; o < 32; o <<= 1) {
+        u64 y = __shfl_down_sync(0xffffffffu, suf, o);
+        if (l + o < 32) suf += y;
+      }
+      u64 cum = es->q_above + (suf - ls);
+      int best = -1;
+      u64 cum_best = 0;
+#pragma unroll
+      for (int q = 7; q >= 0; --q) {
+        cum += loc[q];
+        if (best < 0 && (double)(qt > cum ? qt - cum : 0ull) <= tol_q) {
+          best = 8 * l + q;
+          cum_best = cum;
+        }
+      }
+      int chosen = __reduce_max_sync(0xffffffffu, best);
+      bool none = chosen < 0;
+      if (none) chosen = 0;
+      u64 cb = (best == chosen && !none) ? cum_best : 0ull;
+      u64 hb = (best == chosen && !none) ? es->hist[chosen] : 0ull;
+      for (int o = 16; o > 0; o >>= 1) {
+        cb += __shfl_xor_sync(0xffffffffu, cb, o);
+        hb += __shfl_xor_sync(0xffffffffu, hb, o);
+      }
+      __syncwarp();
+      if (l == 0) {
+        // bins strictly above the chosen one are selected for sure; when no
+        // bin satisfies the tolerance (rounding), take the whole range. The
+        // open last bin of the first pass starts again with bytes.
+        if (octaves) es->qtot = qt;
+        if (!octaves || chosen > 0) es->q_above = none ? es->q_above + all - es->hist[0] : cb - hb;
+        es->digit = chosen;
+      }
+    }
+    __syncthreads();
+    const int digit = es->digit;
+    qtot = es->qtot;
+    if (octaves) {
+      if (digit == 0) continue;
+      pre = (u64)(top - (255 - digit));
+    } else {
+      pre = (pre << w) | (u64)digit;
+    }
+    sh = nsh;
+    if (sh == 0) {
+      tau = pre;
+      break;
+    }
+    if (ncand < 0) {
+      for (int i = tid; i < nlive; i += NT)
+        if ((key_of(i) >> sh) == pre) {
+          const int at = atomicAdd(&es->nlive_chunk, 1);
+          if (at < LIST) es->live_list[at] = i;
+        }
+      __syncthreads();
+      ncand = es->nlive_chunk <= LIST ? es->nlive_chunk : -1;
+      __syncthreads();
+    }
+    if (ncand >= 0 && ncand <= 32) {
+      // at most one a lane: the largest key whose regions and those above
+      // leave a remaining error within the tolerance
+      if (tid < 32) {
+        u64 key = 0, q = 0;
+        bool cand = false;
+        if (lane < ncand) {
+          const int i = es->live_list[lane];
+          key = key_of(i);
+          cand = (key >> sh) == pre;
+          if (cand) q = q_of(i, key);
+        }
+        u64 cum = es->q_above;
+        for (int o = 0; o < ncand; ++o) {
+          const u64 ok = __shfl_sync(0xffffffffu, key, o), oq = __shfl_sync(0xffffffffu, q, o);
+          if (ok >= key) cum += oq;
+        }
+        u64 m = cand && (double)(qtot > cum ? qtot - cum : 0ull) <= tol_q ? key : 0ull;
+        for (int o = 16; o > 0; o >>= 1) {
+          const u64 y = __shfl_xor_sync(0xffffffffu, m, o);
+          m = y > m ? y : m;
+        }
+        if (lane == 0) es->prefix = m ? m : pre << sh;
+      }
+      __syncthreads();
+      tau = es->prefix;
+      break;
+    }
+  }
+
+  // ---------------- ties that the reference form decides --------------
+  if constexpr (REF) {
+    if (!ref && tau != 0ull) {
+      const double kt = __longlong_as_double((long long)tau);
+      const double b0 = kt * (1.0 - TIE_REL), b1 = kt * (1.0 + TIE_REL);
+      if (tid == 0) es->nband = es->nref = 0;
+      __syncthreads();
+      // regions at the cut, where there is more than one
+      int nb = 0;
+      for (int i = tid; i < nlive; i += NT) {
+        const double k = __longlong_as_double((long long)key_of(i));
+        nb += k >= b0 && k <= b1;
+      }
+      if (nb) atomicAdd(&es->nband, nb);
+      __syncthreads();
+      const bool band = es->nband > 1;
+      if (band) {
+        for (int i = tid; i < nlive; i += NT) {
+          const double k = __longlong_as_double((long long)key_of(i));
+          if (k >= b0 && k <= b1 && !(S.split[i] & SPLIT_REF)) S.pend[atomicAdd(&es->nref, 1)] = i;
+        }
+      }
+      __syncthreads();
+      const int nfl = es->nref;
+      __syncthreads();
+      // axes of the regions above them
+      for (int i = tid; i < nlive; i += NT) {
+        const double k = __longlong_as_double((long long)key_of(i));
+        if ((band ? k > b1 : k >= kt) && (S.split[i] & (SPLIT_TIE | SPLIT_AXIS_REF)) == SPLIT_TIE)
+          S.pend[atomicAdd(&es->nref, 1)] = i;
+      }
+      __syncthreads();
+      if (es->nref > 0) {
+        if (tid == 0) {
+          es->npend = es->nref;
+          es->nfull = nfl;
+          es->ref = 1;
+          es->nlive_chunk = 0;
+        }
+        __syncthreads();
+        return;  // all ranks evaluate them, then the cut is drawn again
+      }
+    }
+  }
+
+  // ---------------- compaction: split every region with key >= tau ----
+  // ranks in the order of the regions: each warp counts, then lists, a
+  // contiguous segment
+  const int seg = ((nlive + NT - 1) / NT) * 32;
+  const int lo = min(warp * seg, nlive), hi = min(lo + seg, nlive);
+  int cnt = 0;
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    cnt += __popc(__ballot_sync(0xffffffffu, i < hi && key_of(i) >= tau));
+  }
+  if (lane == 0) es->ired[warp] = cnt;
+  __syncthreads();
+  int rank = 0, ktot = 0;
+  for (int w = 0; w < NT / 32; ++w) {
+    const int c = es->ired[w];
+    rank += w < warp ? c : 0;
+    ktot += c;
+  }
+  if (ktot == 0 || nlive + ktot > S.cap) return finish(ktot == 0 ? 4 : 1);
+  for (int i0 = lo; i0 < hi; i0 += 32) {
+    const int i = i0 + lane;
+    const bool sel = i < hi && key_of(i) >= tau;
+    const unsigned m = __ballot_sync(0xffffffffu, sel);
+    if (sel) S.pend[2 * (rank + __popc(m & ((1u << lane) - 1)))] = i;
+    rank += __popc(m);
+  }
+  __syncthreads();
+  for (int k = tid; k < ktot; k += NT) {
+    const int i = S.pend[2 * k], u = nlive + k;
+    const int d = S.split[i] & SPLIT_AXIS;
+    double v = 1;
+#pragma unroll
+    for (int q = 0; q < DIM; ++q) {
+      double cq = S.cen[(size_t)q * S.cap + i];
+      double hq = S.hw[(size_t)q * S.cap + i];
+      if (q == d) {
+        hq *= 0.5;
+        S.cen[(size_t)q * S.cap + i] = cq - hq;
+        S.hw[(size_t)q * S.cap + i] = hq;
+        S.cen[(size_t)q * S.cap + u] = cq + hq;
+      } else {
+        S.cen[(size_t)q * S.cap + u] = cq;
+      }
+      S.hw[(size_t)q * S.cap + u] = hq;
+      v *= 2 * hq;
+    }
+    S.vol[i] *= 0.5;
+    S.vol[u] = v;
+    S.pend[2 * k + 1] = u;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    es->nlive = nlive + ktot;
+    es->npend = 2 * ktot;
+    es->ref = 0;
+    es->nlive_chunk = 0;
+  }
+}
+
+// out of line: its registers are not the evaluation's
+template <int DIM, int FDIM, int NT, bool REF>
+__device__ __noinline__ void engine_select_call(Slot<DIM, FDIM> S, EngineShared<FDIM>* es, EngineCfg cfg,
+                                                unsigned long long* stage, int stage_bytes, int sweep, int npend,
+                                                int ref) {
+  engine_select<DIM, FDIM, NT, REF>(S, es, cfg, stage, stage_bytes, sweep, npend, ref);
+}
 
 // ---------------------------------------------------------------------------
 // The persistent adaptive-integration kernel body. Policy P provides:
@@ -462,6 +800,7 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
     es0 = cl.map_shared_rank(es, 0);
   }
 
+  const int stage_bytes = (int)((char*)es - recs) & ~15;
   Slot<DIM, FDIM> S;
   S.init(scratch + (size_t)(blockIdx.x / CS) * slot_bytes, cfg.cap);
   const int tid = threadIdx.x;
@@ -683,225 +1022,14 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
         }
       }
       if constexpr (CS > 1) engine_cluster_sync<CS>();
-      // rank 0: totals, convergence, selection and splitting; a stop sets
-      // es->stop and leaves this block
-      if (crank == 0) do {
-      if (tid == 0 && !ref) es->neval += (long long)npend * NP;
-
-      // ---------------- totals and convergence ----------------------------
-      const int nlive = es->nlive;
-      double tv[FDIM], te[FDIM];
-#pragma unroll
-      for (int k = 0; k < FDIM; ++k) {
-        double a = 0, b = 0;
-        for (int i = tid; i < nlive; i += NT) {
-          a += S.val[(size_t)k * S.cap + i];
-          b += S.err[(size_t)k * S.cap + i];
-        }
-        tv[k] = block_sum<NT>(a, es->red);
-        te[k] = block_sum<NT>(b, es->red);
+      // rank 0: totals, convergence, selection and splitting (or a reference
+      // pass, or a stop)
+      if (crank == 0) {
+        if constexpr (REF)
+          engine_select_call<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref);
+        else
+          engine_select<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref);
       }
-      bool conv = converged_check(FDIM, cfg.norm, tv, te, cfg.abs_tol, cfg.rel_tol);
-      if (conv || sweep + 1 >= cfg.max_sweeps) {
-        if (tid == 0) {
-          for (int k = 0; k < FDIM; ++k) {
-            es->V[k] = tv[k];
-            es->E[k] = te[k];
-          }
-          if (!conv) es->status |= 2;
-          es->sweeps = sweep + 1;
-          es->stop = 1;
-        }
-        __syncthreads();
-        break;
-      }
-      // tolerance for the Gladwell pop loop
-      double etot = 0, vabs = 0;
-      bool l1 = !(FDIM == 1 || cfg.norm == TP_NORM_INDIVIDUAL);
-#pragma unroll
-      for (int k = 0; k < FDIM; ++k) {
-        etot += te[k];
-        vabs += fabs(tv[k]);
-      }
-      double tol;
-      if (l1)
-        tol = fmax(cfg.abs_tol, vabs * cfg.rel_tol);
-      else
-        tol = fmax(cfg.abs_tol, fabs(tv[0]) * cfg.rel_tol);
-
-      // ---------------- radix select of the error threshold ---------------
-      // Errors are summed as 62-bit fixed-point fractions of the total error,
-      // so the histogram sums (shared-memory integer atomics) are exact and
-      // independent of the order of the additions.
-      const double qscale = 4.611686018427387904e18 / etot;  // 2^62 / E_tot
-      const double tol_q = tol * qscale;
-      if (tid == 0) {
-        es->prefix = 0ull;
-        es->q_above = 0ull;
-      }
-      for (int pass = 0; pass < 8; ++pass) {
-        const int shift = 56 - 8 * pass;
-        for (int b = tid; b < 256; b += NT) es->hist[b] = 0ull;
-        __syncthreads();
-        const unsigned long long pre = es->prefix;
-        for (int i = tid; i < nlive; i += NT) {
-          unsigned long long key = (unsigned long long)__double_as_longlong(S.emax[i]);
-          if (pass == 0 || (key >> (shift + 8)) == pre) {
-            double es_ = 0;
-#pragma unroll
-            for (int k = 0; k < FDIM; ++k) es_ += S.err[(size_t)k * S.cap + i];
-            atomicAdd(&es->hist[(key >> shift) & 255ull], (unsigned long long)(es_ * qscale));
-          }
-        }
-        __syncthreads();
-        if (tid < 32) {
-          const int l = tid;
-          unsigned long long loc[8];
-          unsigned long long ls = 0;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            loc[q] = es->hist[8 * l + q];
-            ls += loc[q];
-          }
-          // pass 0 histograms every region: its sum is the fixed-point total
-          unsigned long long tot = ls;
-          for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-          __shared__ unsigned long long s_qtot;
-          if (pass == 0 && l == 0) s_qtot = tot;
-          __syncwarp();
-          const unsigned long long qtot = s_qtot;
-          // suffix sum over lanes (lane l: sum of lanes > l)
-          unsigned long long suf = ls;
-          for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long y = __shfl_down_sync(0xffffffffu, suf, o);
-            if (l + o < 32) suf += y;
-          }
-          unsigned long long cum = es->q_above + (suf - ls);
-          int best = -1;
-          unsigned long long cum_best = 0;
-#pragma unroll
-          for (int q = 7; q >= 0; --q) {
-            cum += loc[q];
-            if (best < 0 && (double)(qtot > cum ? qtot - cum : 0ull) <= tol_q) {
-              best = 8 * l + q;
-              cum_best = cum;
-            }
-          }
-          int chosen = __reduce_max_sync(0xffffffffu, best);
-          bool none = chosen < 0;
-          if (none) chosen = 0;
-          unsigned long long cb = (best == chosen && !none) ? cum_best : 0ull;
-          unsigned long long hb = (best == chosen && !none) ? es->hist[chosen] : 0ull;
-          for (int o = 16; o > 0; o >>= 1) {
-            cb += __shfl_xor_sync(0xffffffffu, cb, o);
-            hb += __shfl_xor_sync(0xffffffffu, hb, o);
-          }
-          unsigned long long all = ls;
-          for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
-          if (l == 0) {
-            // bins strictly above the chosen one are selected for sure; when no
-            // bin satisfies the tolerance (rounding), take the whole range
-            es->q_above = none ? es->q_above + all - es->hist[0] : cb - hb;
-            es->prefix = (pre << 8) | (unsigned long long)chosen;
-          }
-        }
-        __syncthreads();
-      }
-      const unsigned long long tau = es->prefix;
-
-      // ---------------- ties that the reference form decides --------------
-      if constexpr (REF) {
-        if (!ref && tau != 0ull) {
-          const double kt = __longlong_as_double((long long)tau);
-          const double b0 = kt * (1.0 - TIE_REL), b1 = kt * (1.0 + TIE_REL);
-          if (tid == 0) es->nband = es->nref = 0;
-          __syncthreads();
-          // regions at the cut, where there is more than one
-          int nb = 0;
-          for (int i = tid; i < nlive; i += NT) nb += S.emax[i] >= b0 && S.emax[i] <= b1;
-          if (nb) atomicAdd(&es->nband, nb);
-          __syncthreads();
-          const bool band = es->nband > 1;
-          if (band) {
-            for (int i = tid; i < nlive; i += NT)
-              if (!(S.split[i] & SPLIT_REF) && S.emax[i] >= b0 && S.emax[i] <= b1)
-                S.pend[atomicAdd(&es->nref, 1)] = i;
-          }
-          __syncthreads();
-          const int nfl = es->nref;
-          __syncthreads();
-          // axes of the regions above them
-          for (int i = tid; i < nlive; i += NT)
-            if ((S.split[i] & (SPLIT_TIE | SPLIT_AXIS_REF)) == SPLIT_TIE && S.emax[i] >= (band ? b0 : kt) &&
-                !(band && S.emax[i] <= b1))
-              S.pend[atomicAdd(&es->nref, 1)] = i;
-          __syncthreads();
-          if (es->nref > 0) {
-            if (tid == 0) {
-              es->npend = es->nref;
-              es->nfull = nfl;
-              es->ref = 1;
-            }
-            __syncthreads();
-            break;  // all ranks evaluate them, then the cut is drawn again
-          }
-        }
-      }
-
-      // ---------------- compaction: split every region with key >= tau ----
-      const int chunk = (nlive + NT - 1) / NT;
-      const int lo = min(tid * chunk, nlive), hi = min(lo + chunk, nlive);
-      int cnt = 0;
-      for (int i = lo; i < hi; ++i)
-        cnt += ((unsigned long long)__double_as_longlong(S.emax[i]) >= tau) ? 1 : 0;
-      int ktot;
-      int rank = block_exclusive_scan<NT>(cnt, es->ired, &ktot);
-      if (ktot == 0 || nlive + ktot > S.cap) {
-        if (tid == 0) {
-          for (int k = 0; k < FDIM; ++k) {
-            es->V[k] = tv[k];
-            es->E[k] = te[k];
-          }
-          es->status |= (ktot == 0) ? 4 : 1;
-          es->sweeps = sweep + 1;
-          es->stop = 1;
-        }
-        __syncthreads();
-        break;
-      }
-      for (int i = lo; i < hi; ++i) {
-        if ((unsigned long long)__double_as_longlong(S.emax[i]) < tau) continue;
-        const int u = nlive + rank;
-        const int d = S.split[i] & SPLIT_AXIS;
-        double v = 1;
-#pragma unroll
-        for (int q = 0; q < DIM; ++q) {
-          double cq = S.cen[(size_t)q * S.cap + i];
-          double hq = S.hw[(size_t)q * S.cap + i];
-          if (q == d) {
-            hq *= 0.5;
-            S.cen[(size_t)q * S.cap + i] = cq - hq;
-            S.hw[(size_t)q * S.cap + i] = hq;
-            S.cen[(size_t)q * S.cap + u] = cq + hq;
-          } else {
-            S.cen[(size_t)q * S.cap + u] = cq;
-          }
-          S.hw[(size_t)q * S.cap + u] = hq;
-          v *= 2 * hq;
-        }
-        S.vol[i] *= 0.5;
-        S.vol[u] = v;
-        S.pend[2 * rank] = i;
-        S.pend[2 * rank + 1] = u;
-        ++rank;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        es->nlive = nlive + ktot;
-        es->npend = 2 * ktot;
-        es->ref = 0;
-      }
-      } while (0);
       engine_cluster_sync<CS>();
       if (es0->stop) break;
       if (!REF || !es0->ref) ++sweep;

@@ -414,8 +414,10 @@ struct HaloProd {
     bool ok = false;
     if constexpr (KIND == 5) {
       const double l1 = exp(x[0]), l2 = exp(x[1]), l5 = exp(x[2]);
-      const double s3 = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(x[3]);
-      const double s6 = l1 * l1 + l5 * l5 + 2 * l1 * l5 * cos(x[4]);
+      // explicit roundings (see rule_combine): l1^2 + l2^2 + 2 l1 l2 cos x3 and
+      // l1^2 + l5^2 + 2 l1 l5 cos x4
+      const double s3 = fma(__dmul_rn(2 * l1, l2), cos(x[3]), fma(l2, l2, __dmul_rn(l1, l1)));
+      const double s6 = fma(__dmul_rn(2 * l1, l5), cos(x[4]), fma(l1, l1, __dmul_rn(l5, l5)));
       if (s3 > 0 && s6 > 0) {
         const double l3 = sqrt(s3), l6 = sqrt(s6);
         if (!(l3 > lmax || l6 > lmax)) {
