@@ -67,7 +67,7 @@ static R node(const Row& r, const EH& e, const double* l, const double* f2t) {
 int main() {
   std::mt19937_64 g(1);
   auto U = [&] { return (double)(g() >> 11) * 0x1p-53; };
-  double ex = 0, lg = 0, mu = 0, ad = 0, rc = 0, to = 0, fr = 0, fx = 0;
+  double sc = 0, ex = 0, lg = 0, mu = 0, ad = 0, rc = 0, to = 0, fr = 0, fx = 0;
   auto rel = [](Q a, Q b) { return (double)fabsl(a / b - 1); };
   for (int i = 0; i < 400000; ++i) {
     int64_t x = (int64_t)((U() * 2 - 1) * 1000 * 0x1p52);
@@ -90,10 +90,15 @@ int main() {
     to = std::max(to, rel((Q)sf_to(a), val(a)));
     const double d = exp2((U() * 2 - 1) * 300);
     fr = std::max(fr, rel(val(sf_from(d)), d));
+    double w = i % 8 ? U() * 7.999 : ldexp((double)(g() % 652), 0) * 0.012271846303085129838 + (U() - 0.5) * 1e-15;
+    if (w < 0) w = 0;
+    int64_t sn, cs;
+    i64_sincos(w, h_i64sin, sn, cs);
+    sc = std::max(sc, (double)std::max(fabsl(ldexpl((Q)sn, -62) - sinl((Q)w)), fabsl(ldexpl((Q)cs, -62) - cosl((Q)w))));
     const double y = (U() * 2 - 1) * exp2(-U() * 60) * 1000;
     fx = std::max(fx, (double)fabsl(ldexpl((Q)i64_fix<52>(y), -52) - (Q)y));
   }
-  printf("exp2 %g\nlog2 %g\nmul %g\nadd %g\nrcp %g\nto_double %g\nfrom_double %g\nfix %g\n", ex, lg, mu, ad, rc, to, fr, fx);
+  printf("sincos %g\nexp2 %g\nlog2 %g\nmul %g\nadd %g\nrcp %g\nto_double %g\nfrom_double %g\nfix %g\n", sc, ex, lg, mu, ad, rc, to, fr, fx);
 
   std::vector<P64Cell> tab(P64_N);
   EH e;

@@ -22,11 +22,12 @@ def report(tmp_path_factory):
 
 
 # (name, bound): relative errors except log2 and the fixed-point conversions
-# (absolute). exp2: truncated products of 2^-64 and the sixth-order term
+# (absolute). sincos: the argument's Q60 rounding and its product with 1/(2 pi),
+# two units of 2^-60 turns = 2^-57.6 radian; exp2: truncated products of 2^-64 and the sixth-order term
 # (2^-8 ln2)^6/720 = 2^-60.6, together below 2^-57.5; log2: (2^-8)^7/(7 ln2) =
 # 2^-58.3 and the Q31 coefficients, below 2^-57; products lose three units of a
 # 62-bit result; a sum keeps at least 58 bits.
-@pytest.mark.parametrize("name,bound", [("exp2", 2.0 ** -57.5), ("log2", 2.0 ** -57), ("mul", 2.0 ** -60),
+@pytest.mark.parametrize("name,bound", [("sincos", 2.0 ** -57.5), ("exp2", 2.0 ** -57.5), ("log2", 2.0 ** -57), ("mul", 2.0 ** -60),
                                         ("add", 2.0 ** -55), ("rcp", 2.0 ** -60), ("to_double", 2.0 ** -52.9),
                                         ("from_double", 0.0), ("fix", 2.0 ** -52.9)])
 def test_functions(report, name, bound):

@@ -796,6 +796,73 @@ __device__ inline bool zcoefs(const TablesDev& t, const CosmoDev& c, double z, R
   return true;
 }
 
+// Node64 row of one arbitrary redshift (zcoefs in the integer arithmetic:
+// every power of ten is one exponent sum). Returns false where integrand_bkappa
+// is zero; N.ok = 0 outside the integer form's domain.
+__device__ inline bool zrow64(const TablesDev& t, const CosmoDev& c, const CosmoK<double>& K, double z,
+                              const uint64_t* __restrict__ ex2, Node64& N) {
+  N.ok = 0;
+  if (z < 1.0e-7) return false;
+  int i0, i1;
+  double w0, w1;
+  interp_mid_w(z / c.zmax * NZ, i0, i1, w0, w1);
+  const double g = t.g[i0] * w0 + t.g[i1] * w1, fK = t.f_K[i0] * w0 + t.f_K[i1] * w1;
+  const double D1 = t.D1[i0] * w0 + t.D1[i1] * w1, rs = t.r_sigma[i0] * w0 + t.r_sigma[i1] * w1;
+  const double ne = t.n_eff[i0] * w0 + t.n_eff[i1] * w1;
+  const double s = rs / fK, hf = c.h / fK, zp = 1.0 + z, ds = D1 * c.sigma8;
+  if (!(K.c64.ok && K.n64[0].ok && z <= 10. && s > 0x1p-27 && s < 0x1p36 && hf > 0x1p-60 && hf < 0x1p60 && ds > 1e-4 &&
+        ds < 1e4 && ne > -5 && ne < 1 && D1 > 1e-30 && D1 < 1e30))
+    return true;
+  auto L = [&](double v) { return i64_log2(v, d_i64tab); };        // Q57
+  auto X = [&](double v) { return i64_fix<52>(v); };               // Q52
+  auto D = [](int64_t q) { return (double)q * 0x1p-57; };
+  auto E = [&](int64_t q) { return i64_exp2(q, ex2); };
+  const int64_t l2s = L(s), l2D = L(D1), l2zp = L(zp);
+  const double L10 = LOG2_10, ls = D(L(ds)) * 0.30102999566398119521, lz = D(l2zp);
+  N.l2s = l2s;
+  N.l2hf = L(hf);
+  const int64_t s52 = l2s >> 5;
+  // Q59 (and Q60) of a power; too large a one leaves the row to the FP64 form
+  bool ok = true;
+  auto Q = [&](double v, int q) {
+    const Sf r = E(X(v));
+    ok = ok && r.e < -q;  // below 2^(64 - q)
+    return i64_shr(r.m, -q - r.e);
+  };
+  N.l2anr = K.n64[0].l2anr;
+  N.anc = Q(L10 * (0.182 + 0.57 * ne), 59);
+  N.ana = X(L10 * (-2.167 + ls * (-2.944 + ls * (-1.106 + ls * -2.865))));
+  N.ala = X(L10 * (-4.348 + ne * (-3.006 + ne * -0.5745)));
+  N.ald = Q(L10 * (-0.9 + 0.2 * ne) + 1.7320208456446193, 59);  // + log2(log2(10))
+  N.betab = Q(L10 * (-1.731 + ne * (-2.845 + ne * (-1.4995 + ne * -0.2811))), 60);
+  N.l2bn = X(L10 * (-3.428 + ls * (-2.681 + ls * (1.624 + ls * -0.095))));
+  N.mun = Q(L10 * (15.312 + ne * (22.977 + ne * (10.9579 + ne * 1.6586))), 59);
+  N.nun = Q(L10 * (1.347 + ne * (1.246 + ne * 0.4525)), 59);
+  N.kmn = (int64_t)((uint64_t)X(L10 * (-2.605 + ls * (-2.434 + ls * 5.71))) - (N.mun >> 1));
+  N.knn = (int64_t)((uint64_t)X(L10 * (-4.468 + ls * (-3.08 + ls * 1.035))) - (N.nun >> 1));
+  Sf v = E(X(L10 * (0.159 - 1.107 * ne)) + s52);
+  N.cns = v.m, N.ecns = v.e;
+  v = sf_norm(sf_mul(sf_norm(sf_mul(v, v)), v));
+  N.cns3 = v.m, N.ecns3 = v.e;
+  v = E(X(L10 * (-10.533 + ne * (-16.838 + ne * (-9.3048 + ne * -1.8263)))) + 2 * s52 + 2 * (l2D >> 5));
+  N.fn = v.m, N.efn = v.e;
+  v = sf_from(D1 * D1);
+  N.d1 = v.m, N.ed1 = v.e;
+  v = E(X(L10 * (-1.118 - 0.394 * ne)) + 2 * s52);
+  N.hn = v.m, N.ehn = v.e;
+  v = E(X(L10 * (2.787 + ne * (2.405 + ne * 0.4577))) + s52);
+  N.gn = v.m, N.egn = v.e;
+  v = E(3 * (X(L10 * (0.071 - 0.433 * ne)) + s52));
+  N.pn3 = v.m, N.epn3 = v.e;
+  const double omz = c.om / (c.om + c.ow * sf_to(E(X(3. * c.w * lz))));
+  N.ens = sf_to(E(X(L10 * (-0.632 + 0.646 * ne)) + s52));
+  N.dns = sf_to(E(X(L10 * (-0.483 + 0.892 * ls - 0.086 * omz)) + s52));
+  const double Ez = sqrt(c.om * zp * zp * zp + c.ow * sf_to(E(X(3 * (1.0 + c.w) * lz)))), gz = g * zp;
+  N.w = gz * gz * gz / (fK * Ez);
+  N.ok = ok;
+  return true;
+}
+
 __device__ __forceinline__ double uhat(double eta) {
   double t = 0.5 * eta * eta;
   return t * exp(-t);

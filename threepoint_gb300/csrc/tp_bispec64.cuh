@@ -236,25 +236,41 @@ TP_HD Sf p64_eval(const P64Cell* __restrict__ tab, uint64_t lkb, const uint64_t*
   return i64_exp2((int64_t)(lkb >> 3) - h, ex2);
 }
 
-// B of one node (weight not applied); T.ok, N.ok and the cosmology's ok hold
-TP_HD double bispec64(const Node64& N, const Tri64& T, const Cosmo64& C, const uint64_t* __restrict__ ex2) {
-  // a_n, alpha_n, beta_n of this triangle (B7)
-  const Sf sa = i64_exp2(N.l2anr - (int64_t)i64_mulhi(T.nlr, N.anc), ex2);
+// a_n, alpha_n, beta_n of a triangle shape (B7) as the exponents' coefficients
+// and offsets: 2^ka (64 q)^al = a_n q^al
+struct Shape64 {
+  uint64_t al, be;  // Q59
+  uint64_t ka, kb;  // Q52, modulo 2^64
+};
+TP_HD Shape64 shape64(const Node64& N, uint64_t nlr, uint64_t r2, uint64_t pr2, uint64_t amax,
+                      const uint64_t* __restrict__ ex2) {
+  Shape64 h;
+  const Sf sa = i64_exp2(N.l2anr - (int64_t)i64_mulhi(nlr, N.anc), ex2);
   const int64_t l2an = N.ana - (int64_t)i64_shr(sa.m, -52 - sa.e);
-  const Sf sl = i64_exp2(N.ala + (int64_t)i64_mulhi(T.r2, N.ald), ex2);
-  uint64_t al = sl.e < -63 ? i64_shr(sl.m, -59 - sl.e) : ~0ull;
-  al = al < C.amax ? al : C.amax;
-  const uint64_t be = i64_mulhi(N.betab, T.pr2);
-  const uint64_t ka = (uint64_t)l2an - (al >> 1), kb = (uint64_t)N.l2bn - (be >> 1);
+  const Sf sl = i64_exp2(N.ala + (int64_t)i64_mulhi(r2, N.ald), ex2);
+  const uint64_t al = sl.e < -63 ? i64_shr(sl.m, -59 - sl.e) : ~0ull;
+  h.al = al < amax ? al : amax;
+  h.be = i64_mulhi(N.betab, pr2);
+  h.ka = (uint64_t)l2an - (h.al >> 1);
+  h.kb = (uint64_t)N.l2bn - (h.be >> 1);
+  return h;
+}
+
+// B of one node (weight not applied) for a triangle shape and its sides:
+// S.side(i, lgb, l, l2, l3) gives side i, S.product() ell1 ell2 ell3
+template <class S>
+TP_HD double bispec64_core(const Node64& N, const Shape64& h, const S& src, const double* f2t,
+                           const P64Cell* __restrict__ ptab, const uint64_t* __restrict__ ex2) {
   Sf den1 = sf_one();
   double P[3], f[3], e3 = 1.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const Tri64::Side& S = T.s[i];
-    const uint64_t lq = S.lgb + (uint64_t)N.l2s;
-    const Sf l = {S.m, S.e}, l2 = {S.m2, S.e2}, l3 = {S.m3, S.e3};
+    uint64_t lgb;
+    Sf l, l2, l3;
+    src.side(i, lgb, l, l2, l3);
+    const uint64_t lq = lgb + (uint64_t)N.l2s;
     // 1-halo denominators (B4)
-    const Sf d = sf_add(i64_exp2((int64_t)(i64_mulhi(lq, al) + ka), ex2), i64_exp2((int64_t)(i64_mulhi(lq, be) + kb), ex2));
+    const Sf d = sf_add(i64_exp2((int64_t)(i64_mulhi(lq, h.al) + h.ka), ex2), i64_exp2((int64_t)(i64_mulhi(lq, h.be) + h.kb), ex2));
     const Sf cq1 = sf_add(sf_mul({N.cns, N.ecns}, l), sf_one());
     den1 = sf_norm(sf_mul(den1, sf_mul(d, cq1)));
     // 3-halo side (B5, B9) over the common denominator
@@ -264,19 +280,34 @@ TP_HD double bispec64(const Node64& N, const Tri64& T, const Cosmo64& C, const u
     const Sf mq = sf_add(i64_exp2((int64_t)(i64_mulhi(lq, N.mun) + (uint64_t)N.kmn), ex2),
                          i64_exp2((int64_t)(i64_mulhi(lq, N.nun) + (uint64_t)N.knn), ex2));
     const Sf M = sf_norm(sf_mul(mq, sf_add(x3, sf_one())));
-    const Sf pl = p64_eval(C.p, S.lgb + (uint64_t)N.l2hf, ex2);
+    const Sf pl = p64_eval(ptab, lgb + (uint64_t)N.l2hf, ex2);
     const Sf nm = sf_add(sf_mul(x3, den), sf_mul(sf_mul(num, pl), M));
     P[i] = sf_to(sf_mul(nm, sf_rcp(sf_mul(den, M))));
     const double ld = sf_to(l);
-    f[i] = fma(N.dns, ld, T.f2t[i == 2 ? 0 : i + 1]);
+    f[i] = fma(N.dns, ld, f2t[i == 2 ? 0 : i + 1]);
     e3 *= fma(N.ens, ld, 1.0);
   }
-  const double b1 = sf_to(sf_mul(sf_mul({N.cns3, N.ecns3}, {T.lp, T.elp}), sf_rcp(den1)));
+  const double b1 = sf_to(sf_mul(sf_mul({N.cns3, N.ecns3}, src.product()), sf_rcp(den1)));
   // F2 of the pairs (0,1), (1,2), (2,0): f[2], f[0], f[1]
   double b3 = f[2] * (P[0] * P[1]);
   b3 = fma(f[0], P[1] * P[2], b3);
   b3 = fma(f[1], P[2] * P[0], b3);
   return fma(2.0 * b3, sf_to(sf_rcp(sf_from(e3))), b1);
+}
+
+struct TriSides64 {
+  const Tri64& T;
+  TP_HD void side(int i, uint64_t& lgb, Sf& l, Sf& l2, Sf& l3) const {
+    const Tri64::Side& S = T.s[i];
+    lgb = S.lgb;
+    l = {S.m, S.e}, l2 = {S.m2, S.e2}, l3 = {S.m3, S.e3};
+  }
+  TP_HD Sf product() const { return {T.lp, T.elp}; }
+};
+
+// T.ok, N.ok and the cosmology's ok hold
+TP_HD double bispec64(const Node64& N, const Tri64& T, const Cosmo64& C, const uint64_t* __restrict__ ex2) {
+  return bispec64_core(N, shape64(N, T.nlr, T.r2, T.pr2, C.amax, ex2), TriSides64{T}, T.f2t, C.p, ex2);
 }
 
 }  // namespace tp

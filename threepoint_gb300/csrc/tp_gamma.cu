@@ -116,15 +116,35 @@ struct GammaPolicy {
   static constexpr int G = 8;     // groups of 4 Ogata nodes
   static constexpr int KPG = 4;
   static constexpr int CH = 4;    // regions per chunk (records are large)
-  // FP64: the per-point NC_* coefficients (bispec_eval); FP32: the folded
-  // NF_* row (bispec_fast_row), an odd number of words (57) per record
-  struct RecD {
+  // FP64: the per-point node coefficients; FP32: the folded NF_* row
+  // (bispec_fast_row), an odd number of words (57) per record
+  struct RefD {
     double zc[NC_COUNT];
     Tri<double> tri;  // unit-scale triangle (cos psi, sin psi, ell3/psi_k)
     double invA[3], l2A[3];
     double cre[3], cim[3];
     double bmin;
     int live;
+  };
+  struct FastD {
+    Node64 N;
+    Shape64 h;
+    uint64_t lgb[3], m[3], lp;  // log2 ell + 64 (Q57), mantissas of ell_i and ell1 ell2 ell3 at unit scale
+    int e[3], elp;
+    double f2t[3];
+    int64_t l2ia[3];  // log2 (1 / A_j), Q57
+    uint64_t iam[3];  // 1 / A_j
+    int iae[3], pad;
+    double cre[3], cim[3];
+  };
+  // FP64: the integer-arithmetic form, or (f64form) the FP64 instructions'; 59
+  // 64-bit words, conflict-free across lanes
+  struct RecD {
+    union {
+      FastD f;
+      RefD d;
+    };
+    int live, f64form;
   };
   struct RecF {
     float nf[NCP];
@@ -140,7 +160,18 @@ struct GammaPolicy {
   static constexpr int PD = 2;
   static constexpr int NS = 1;
   __device__ static int slot(int) { return 0; }
-  static constexpr size_t PSMEM = sizeof(CosmoK<R>) + 64;
+  // the set-up below and its reference form (the trigonometric one) decide
+  // together where the cubature cuts between tied regions
+  static constexpr bool REF = true;
+  int ref = 0;
+  // per job: sides and half interior angle of term j, its constant phase
+  struct Term {
+    double a, b, ch, sh, ce, se;
+  };
+  static constexpr size_t EX2_BYTES = sizeof(R) == 8 ? sizeof(I64Tables::ex2) : 0;
+  static constexpr size_t PSMEM = EX2_BYTES + sizeof(CosmoK<R>) + 3 * sizeof(Term) + 64;
+  const uint64_t* s_ex2;
+  Term* s_term;
 
   GammaJobs J;
   const TablesDev* tab;
@@ -158,8 +189,13 @@ struct GammaPolicy {
   double zmax;
 
   __device__ void begin_job(int job, char* psmem, double* xmin, double* xmax) {
-    s_ck = (CosmoK<R>*)psmem;
+    s_ex2 = (const uint64_t*)psmem;
+    s_term = (Term*)(psmem + EX2_BYTES);
+    s_ck = (CosmoK<R>*)(psmem + EX2_BYTES + 3 * sizeof(Term));
     if (threadIdx.x == 0) *s_ck = ck[cosmo];
+    if constexpr (sizeof(R) == 8) {
+      for (int i = threadIdx.x; i < 256; i += blockDim.x) ((uint64_t*)psmem)[i] = d_i64tab.ex2[i];
+    }
     const int t = J.tri[job], c = J.comp[job];
     double a = J.x[3 * t], b = J.x[3 * t + 1], d = J.x[3 * t + 2];
     which = c == 0 ? 0 : 1;
@@ -178,6 +214,20 @@ struct GammaPolicy {
     p1 = interior_angle(x2, x3, x1);
     p2 = interior_angle(x3, x1, x2);
     p3 = interior_angle(x1, x2, x3);
+    if (threadIdx.x < 3) {
+      const int j = threadIdx.x;
+      Term t;
+      if (which == 0) {
+        t.a = xs[j][0], t.b = xs[j][1];
+        sincos(0.5 * vp[j], &t.sh, &t.ch);
+        sincos(ph0[j], &t.se, &t.ce);
+      } else {
+        t.a = xs[(j + 1) % 3][0], t.b = xs[(j + 1) % 3][1];
+        sincos(0.5 * (j == 0 ? p1 : j == 1 ? p2 : p3), &t.sh, &t.ch);
+        sincos(j == 0 ? p3 - p2 : j == 1 ? p3 - p1 - 2 * p2 : p1 - p2 + 2 * p3, &t.se, &t.ce);
+      }
+      s_term[j] = t;
+    }
     zmax = cosm[cosmo].zmax;
     xmin[0] = 0;
     xmin[1] = 0;
@@ -190,18 +240,20 @@ struct GammaPolicy {
 
   __device__ bool is_live(const char* recp) const { return ((const Rec*)recp)->live != 0; }
 
-  __device__ bool setup(int p, const double* x, char* recp) {
-    (void)p;
-    Rec& r = *(Rec*)recp;
+  // the reference form's point: the angles of gamma.cu:419-529 themselves; a
+  // function of its own, so that what the compiler contracts in it does not
+  // depend on the fast form
+  template <class Q>
+  __device__ __noinline__ bool setup_ref(const double* x, Q& q) const {
     const double z = x[0], phi = x[1], psi = x[2];
     if constexpr (sizeof(R) == 4) {
       float zc[NC_COUNT];
-      r.live = zcoefs<float>(tab[cosmo], cosm[cosmo], z, zc);
-      if (r.live) nf_from_nc(zc, r.nf);
+      q.live = zcoefs<float>(tab[cosmo], cosm[cosmo], z, zc);
+      if (q.live) nf_from_nc(zc, q.nf);
     } else {
-      r.live = zcoefs<R>(tab[cosmo], cosm[cosmo], z, r.zc);
+      q.live = zcoefs<R>(tab[cosmo], cosm[cosmo], z, q.zc);
     }
-    if (!r.live) return false;
+    if (!q.live) return false;
     // the geometry is evaluated in double: a few dozen operations per point
     // against 96 bispectra
     double cp = cos(psi), sp = sin(psi), s2p = sin(2 * psi), c2p = cos(2 * psi);
@@ -209,17 +261,17 @@ struct GammaPolicy {
     double bb = 0.5 * atan2(c2p * sph, cph + s2p);  // betabar, gamma.cu:524-529
     double b3s = cp * cp + sp * sp + 2 * cp * sp * cph;
     double b3 = b3s <= 0 ? 0.0 : sqrt(b3s);
-    r.bmin = (R)fmin(cp, fmin(sp, b3));
+    q.bmin = (R)fmin(cp, fmin(sp, b3));
     if (!(b3 > 0 && cp > 0 && sp > 0)) {
-      r.live = 0;
+      q.live = 0;
       return false;
     }
     if constexpr (sizeof(R) == 4) {
       Tri<float> t;
       make_tri_phi_f((float)cp, (float)sp, (float)cph, (float)b3, t);
-      trif_from_tri(t, r.tri);
+      trif_from_tri(t, q.tri);
     } else {
-      make_tri<R>(cp, sp, b3, r.tri);
+      make_tri<R>(cp, sp, b3, q.tri);
     }
     if (which == 0) {
       const double xs[3][2] = {{x1, x2}, {x2, x3}, {x3, x1}};
@@ -230,10 +282,10 @@ struct GammaPolicy {
         double al = atan2((cp * b - sp * a) * sin(ang / 2), (cp * b + sp * a) * cos(ang / 2));
         double phase = ph0[j] - 6 * al + 2 * bb;
         double mag = s2p * PI / (A * A * A * A);
-        r.invA[j] = (R)(1.0 / A);
-        r.l2A[j] = (R)log2(A);
-        r.cre[j] = (R)(mag * cos(phase));
-        r.cim[j] = (R)(mag * sin(phase));
+        q.invA[j] = (R)(1.0 / A);
+        q.l2A[j] = (R)log2(A);
+        q.cre[j] = (R)(mag * cos(phase));
+        q.cim[j] = (R)(mag * sin(phase));
       }
     } else {
       // term order as full_integrand_gamma1: j=0 -> A1, 1 -> A2, 2 -> A3
@@ -252,18 +304,253 @@ struct GammaPolicy {
       ph[2] = p1 - p2 + 2 * p3 + 2 * (bb - phi - alv[2]);
       for (int j = 0; j < 3; ++j) {
         double mag = s2p * PI / (Av[j] * Av[j] * Av[j] * Av[j]);
-        r.invA[j] = (R)(1.0 / Av[j]);
-        r.l2A[j] = (R)log2(Av[j]);
-        r.cre[j] = (R)(mag * cos(ph[j]));
-        r.cim[j] = (R)(mag * sin(ph[j]));
+        q.invA[j] = (R)(1.0 / Av[j]);
+        q.l2A[j] = (R)log2(Av[j]);
+        q.cre[j] = (R)(mag * cos(ph[j]));
+        q.cim[j] = (R)(mag * sin(ph[j]));
       }
     }
     return true;
   }
 
+  __device__ bool setup(int p, const double* x, char* recp) {
+    (void)p;
+    Rec& r = *(Rec*)recp;
+    if constexpr (sizeof(R) == 4) {
+      return ref ? setup_ref(x, r) : setup_f32(x, r);
+    } else {
+      r.f64form = ref || !setup_f64(x, r);
+      if (r.f64form) {
+        const bool live = setup_ref(x, r.d);
+        r.live = live;
+      }
+      return r.live;
+    }
+  }
+
+  // The point geometry without inverse functions. With c, s = cos, sin of
+  // phi/2, the side of term j is the complex number
+  //   w = (cos psi b + sin psi a) cos(phi/2 + vp/2) + i (cos psi b - sin psi a) sin(phi/2 + vp/2),
+  // |w| = A_j and arg w = alpha_j (gamma.cu:491-522), and betabar is -arg of
+  //   v = (cos psi + sin psi) c + i (sin psi - cos psi) s,  |v| = ell3 / psi_k,
+  // so every phase is a product of unit complex numbers. Two sincos and three
+  // square roots are left of ~35 FP64 functions a point, which took 4/5 of the
+  // FP32 form's time; A_j as a sum of squares does not cancel.
+  struct Geo {
+    double cp, sp, cph, b3;
+    double A2[3], cre[3], cim[3], mag[3], k2[3];  // k2: (cos psi b + sin psi a)^2
+    double b2;
+  };
+  __device__ __forceinline__ bool geometry(double phi, double psi, Geo& G) const {
+    double c, s;
+    if constexpr (sizeof(R) == 4) {  // 2^-60 absolute, on the integer pipe
+      int64_t qs, qc;
+      i64_sincos(psi, d_i64sin, qs, qc);
+      G.sp = i64_q62(qs), G.cp = i64_q62(qc);
+      i64_sincos(0.5 * phi, d_i64sin, qs, qc);
+      s = i64_q62(qs), c = i64_q62(qc);
+    } else {
+      sincos(psi, &G.sp, &G.cp);
+      sincos(0.5 * phi, &s, &c);
+    }
+    const double cp = G.cp, sp = G.sp, s2p = 2 * sp * cp;
+    const double vr = (cp + sp) * c, vi = (cp - sp) * s;  // conj v
+    const double b2 = vr * vr + vi * vi;
+    G.cph = 1 - 2 * s * s;
+    G.b2 = b2;
+    G.b3 = sqrt(b2);
+    if (!(G.b3 > 0 && cp > 0 && sp > 0)) return false;
+    const double ib2 = 1 / b2;
+    const double ur = (vr * vr - vi * vi) * ib2, ui = 2 * vr * vi * ib2;  // e^(2 i betabar)
+    const double fr = G.cph, fi = 2 * s * c;                             // e^(i phi)
+    const double f2r = fr * fr - fi * fi, f2i = 2 * fr * fi;             // e^(2 i phi)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const Term& t = s_term[j];
+      const double ca = c * t.ch - s * t.sh, sa = s * t.ch + c * t.sh;  // (phi + vp) / 2
+      const double wr = (cp * t.b + sp * t.a) * ca, wi = (cp * t.b - sp * t.a) * sa;
+      const double A2 = wr * wr + wi * wi, iA2 = 1 / A2;
+      G.A2[j] = A2;
+      G.k2[j] = (cp * t.b + sp * t.a) * (cp * t.b + sp * t.a);
+      const double qr = (wr * wr - wi * wi) * iA2, qi = -2 * wr * wi * iA2;  // e^(-2 i alpha)
+      double er, ei;
+      if (which == 0) {
+        // ph0 - 6 alpha + 2 betabar
+        const double q2r = qr * qr - qi * qi, q2i = 2 * qr * qi;
+        const double q3r = q2r * qr - q2i * qi, q3i = q2r * qi + q2i * qr;
+        er = q3r * ur - q3i * ui;
+        ei = q3r * ui + q3i * ur;
+      } else {
+        // j = 0: -2 (betabar + alpha); 1: 2 (betabar + phi - alpha); 2: 2 (betabar - phi - alpha)
+        const double br = ur, bi = j == 0 ? -ui : ui;
+        er = qr * br - qi * bi;
+        ei = qr * bi + qi * br;
+        if (j > 0) {
+          const double gi = j == 1 ? f2i : -f2i, xr = er * f2r - ei * gi;
+          ei = er * gi + ei * f2r;
+          er = xr;
+        }
+      }
+      const double mag = s2p * PI * iA2 * iA2;
+      G.mag[j] = mag;
+      G.cre[j] = mag * (er * t.ce - ei * t.se);
+      G.cim[j] = mag * (er * t.se + ei * t.ce);
+    }
+    return true;
+  }
+
+  // the redshift and shape rows of a point as the reference form makes them
+  static __device__ __noinline__ bool zrow_f32(const TablesDev& t, const CosmoDev& c, double z, float* nf) {
+    float zc[NC_COUNT];
+    const bool live = zcoefs<float>(t, c, z, zc);
+    if (live) nf_from_nc(zc, nf);
+    return live;
+  }
+  static __device__ __noinline__ void tri_f32(float cp, float sp, float cph, float b3, TriF& F) {
+    Tri<float> t;
+    make_tri_phi_f(cp, sp, cph, b3, t);
+    trif_from_tri(t, F);
+  }
+
+  // The FP32 record rounds the geometry's doubles. Where a value lies so near
+  // the middle of two floats that the rounding error of this geometry or of
+  // the reference form's (which grows with the cancellation in A_j and betabar)
+  // could reach it, the point takes the reference form, so that both make the
+  // same floats: ~1 point in 3000. ulps: that error in units of 2^-53 of v.
+  static __device__ __forceinline__ bool rounds_alike(double v, int ulps) {
+    const int low = __double2loint(v) & 0x1fffffff, d = low - 0x10000000;
+    return (d < 0 ? -d : d) > ulps;
+  }
+  // the same for an absolute error of ulps units of 2^-53 |scale|
+  static __device__ __forceinline__ bool rounds_alike(double v, double scale, int ulps) {
+    const int de = ((__double2hiint(scale) >> 20) & 2047) - ((__double2hiint(v) >> 20) & 2047) + 1;
+    return de < 20 && rounds_alike(v, de > 0 ? ulps << de : ulps);
+  }
+
+  __device__ bool setup_f32(const double* x, RecF& r) const {
+    Geo G;
+    r.live = zrow_f32(tab[cosmo], cosm[cosmo], x[0], r.nf);
+    if (!r.live) return false;
+    if (!geometry(x[1], x[2], G)) return setup_ref(x, r);
+    const double ib2 = 1 / G.b2;
+    bool same = ib2 < 1e4 && rounds_alike(G.cp, 1.0, 64) && rounds_alike(G.sp, 1.0, 64) &&
+                rounds_alike(G.cph, 1.0, 64) && rounds_alike(G.b3, 64 + (int)(16 * ib2));
+    r.bmin = (float)fmin(G.cp, fmin(G.sp, G.b3));
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double A2 = G.A2[j], kap = G.k2[j] / A2;
+      same = same && kap < 1e3 && A2 > 1e-60 && A2 < 1e60;
+      const int m = 128 + (int)(64 * fmin(kap, 1e3) + 16 * fmin(ib2, 1e4));
+      const int64_t la = i64_log2(A2, d_i64tab) / 2;  // log2 A_j, Q57
+      const double l2 = (double)la * 0x1p-57, ia = sf_to(i64_exp2(-(la >> 5), d_i64tab.ex2));
+      same = same && rounds_alike(ia, m) && rounds_alike(l2, 2.0, m) && rounds_alike(G.cre[j], G.mag[j], m) &&
+             rounds_alike(G.cim[j], G.mag[j], m);
+      r.invA[j] = (float)ia;
+      r.l2A[j] = (float)l2;
+      r.cre[j] = (float)G.cre[j];
+      r.cim[j] = (float)G.cim[j];
+    }
+    if (!same) return setup_ref(x, r);
+    tri_f32((float)G.cp, (float)G.sp, (float)G.cph, (float)G.b3, r.tri);
+    return true;
+  }
+
+  // false: outside the integer form's domain
+  __device__ bool setup_f64(const double* x, RecD& r) const {
+    FastD& f = r.f;
+    const CosmoK<double>& K = *(const CosmoK<double>*)s_ck;
+    r.live = 0;
+    if (!zrow64(tab[cosmo], cosm[cosmo], K, x[0], s_ex2, f.N)) return true;
+    if (!f.N.ok) return false;
+    Geo G;
+    if (!geometry(x[1], x[2], G)) return true;
+    const double l[3] = {G.cp, G.sp, G.b3};
+    f2_trees(G.cp, G.sp, G.b3, f.f2t);
+    double a = l[0], b = l[1], c = l[2], t;
+    if (a < b) { t = a; a = b; b = t; }
+    if (a < c) { t = a; a = c; c = t; }
+    if (b < c) { t = b; b = c; c = t; }
+    if (!(c > 1e-12)) return false;
+    int64_t lmin = 0, lmax = 0, amin = 0, amax = 0;
+    Sf lp = sf_one();
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int64_t g = i64_log2(l[i], d_i64tab);
+      lmin = i == 0 || g < lmin ? g : lmin;
+      lmax = i == 0 || g > lmax ? g : lmax;
+      const Sf v = sf_from(l[i]);
+      f.lgb[i] = (uint64_t)g + (64ull << 57);
+      f.m[i] = v.m, f.e[i] = v.e;
+      lp = sf_norm(sf_mul(lp, v));
+      const double A2 = G.A2[i];
+      if (!(A2 > 1e-60 && A2 < 1e60)) return false;
+      const int64_t la = i64_log2(A2, d_i64tab) / 2;
+      f.l2ia[i] = -la;
+      amin = i == 0 || la < amin ? la : amin;
+      amax = i == 0 || la > amax ? la : amax;
+      const Sf ia = sf_norm(sf_from(1.0 / sqrt(A2)));
+      f.iam[i] = ia.m, f.iae[i] = ia.e;
+      f.cre[i] = G.cre[i], f.cim[i] = G.cim[i];
+    }
+    f.lp = lp.m, f.elp = lp.e;
+    // every ell of the 96 evaluations inside the integer form's domain
+    const double lo = (double)(lmin - amax) * 0x1p-57 + c_og.l2psi[which][1];
+    const double hi = (double)(lmax - amin) * 0x1p-57 + c_og.l2psi[which][PREC_K - 1];
+    const double hf = (double)f.N.l2hf * 0x1p-57, ss = (double)f.N.l2s * 0x1p-57;
+    if (!(lo > -33.2 && hi < 40 && lo + hf > P64_LO + 0.01 && hi + hf < P64_HI - 0.01 && lo + ss > -63 && hi + ss < 63))
+      return false;
+    const double r2 = (b + c - a) / a;
+    const Sf pr = i64_exp2(i64_fix<52>(LOG2_10 * 0.007 * r2), s_ex2);
+    f.h = shape64(f.N, (uint64_t)(lmax - lmin), (uint64_t)i64_fix<57>(r2 * r2), i64_shr(pr.m, -63 - pr.e), K.c64.amax,
+                  s_ex2);
+    r.live = 1;
+    return true;
+  }
+
+  // a point's triangle scaled by sc
+  struct Scaled {
+    const FastD& f;
+    Sf sc;
+    uint64_t l2sc;
+    __device__ __forceinline__ void side(int i, uint64_t& lgb, Sf& l, Sf& l2, Sf& l3) const {
+      lgb = f.lgb[i] + l2sc;
+      l = sf_norm(sf_mul({f.m[i], f.e[i]}, sc));
+      l2 = sf_norm(sf_mul(l, l));
+      l3 = sf_norm(sf_mul(l2, l));
+    }
+    __device__ __forceinline__ Sf product() const {
+      return sf_norm(sf_mul({f.lp, f.elp}, sf_norm(sf_mul(sf_norm(sf_mul(sc, sc)), sc))));
+    }
+  };
+
+  // the reference form's group (FP64 instructions)
+  static __device__ __noinline__ void group_ref(const RefD& r, int og, int g, const CosmoK<R>& K, double* pv) {
+    KSum<R> are, aim;
+    const R* zc = r.zc;
+    const R s = zc[NC_S], l2s = zc[NC_L2S], hf = zc[NC_HF], l2hf = zc[NC_L2HF], W = zc[NC_W];
+    for (int kk = 0; kk < KPG; ++kk) {
+      const int k = 1 + g * KPG + kk;
+      const R psik = (R)c_og.psi[og][k], l2psik = (R)c_og.l2psi[og][k], prodk = (R)c_og.prod[og][k];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        R sc = psik * r.invA[j];
+        if (r.bmin * sc <= (R)1.0e-10) continue;  // integrand_bkappa: ell <= 1e-10 -> 0
+        R l2sc = l2psik - r.l2A[j];
+        R B = bispec_eval<R>(zc, 1, s * sc, l2s + l2sc, hf * sc, l2hf + l2sc, r.tri, K);
+        R v = W * B;
+        if (v != v) v = (R)0;  // NaN -> 0 (bispectrum.cu:327-331)
+        v *= prodk;
+        are.add(r.cre[j] * v);
+        aim.add(r.cim[j] * v);
+      }
+    }
+    pv[0] = (double)are.s;
+    pv[1] = (double)aim.s;
+  }
+
   __device__ void group(const char* recp, int g, double* pv) {
     const Rec& r = *(const Rec*)recp;
-    const CosmoK<R> K = *s_ck;
+    typename std::conditional<sizeof(R) == 4, const CosmoK<R>, const CosmoK<R>&>::type K = *s_ck;
     const int og = which;
     KSum<R> are, aim;
     if constexpr (sizeof(R) == 4) {
@@ -285,22 +572,21 @@ struct GammaPolicy {
         }
       }
     } else {
-      const R* zc = r.zc;
-      const R s = zc[NC_S], l2s = zc[NC_L2S], hf = zc[NC_HF], l2hf = zc[NC_L2HF], W = zc[NC_W];
+      if (r.f64form) return group_ref(r.d, og, g, K, pv);
+      const FastD& f = r.f;
+#pragma unroll 1
       for (int kk = 0; kk < KPG; ++kk) {
         const int k = 1 + g * KPG + kk;
-        const R psik = (R)c_og.psi[og][k], l2psik = (R)c_og.l2psi[og][k], prodk = (R)c_og.prod[og][k];
-#pragma unroll
+        const Sf psi = sf_from(c_og.psi[og][k]);
+        const uint64_t l2psi = (uint64_t)i64_fix<57>(c_og.l2psi[og][k]);
+        const double wk = f.N.w * c_og.prod[og][k];
+#pragma unroll 1
         for (int j = 0; j < 3; ++j) {
-          R sc = psik * r.invA[j];
-          if (r.bmin * sc <= (R)1.0e-10) continue;  // integrand_bkappa: ell <= 1e-10 -> 0
-          R l2sc = l2psik - r.l2A[j];
-          R B = bispec_eval<R>(zc, 1, s * sc, l2s + l2sc, hf * sc, l2hf + l2sc, r.tri, K);
-          R v = W * B;
-          if (v != v) v = (R)0;  // NaN -> 0 (bispectrum.cu:327-331)
-          v *= prodk;
-          are.add(r.cre[j] * v);
-          aim.add(r.cim[j] * v);
+          const Scaled S = {f, sf_norm(sf_mul(psi, {f.iam[j], f.iae[j]})), l2psi + (uint64_t)f.l2ia[j]};
+          double v = wk * bispec64_core(f.N, f.h, S, f.f2t, K.c64.p, s_ex2);
+          if (v != v) v = 0;  // NaN -> 0 (bispectrum.cu:327-331)
+          are.add(f.cre[j] * v);
+          aim.add(f.cim[j] * v);
         }
       }
     }
@@ -336,7 +622,7 @@ struct GammaPolicy {
 
 // CS > 1: one cluster of CS CTAs per integral (cooperative adaptive_body)
 template <typename R, int NT, int CS>
-__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? TP_GAMMA_MINB : 1) k_gamma(GammaPolicy<R> pol_in, int njobs, int* job_counter, EngineCfg cfg,
+__global__ void __launch_bounds__(NT, sizeof(R) == 4 ? TP_GAMMA_MINB : 2) k_gamma(GammaPolicy<R> pol_in, int njobs, int* job_counter, EngineCfg cfg,
                                               char* scratch, size_t slot_bytes) {
   GammaPolicy<R> pol = pol_in;
   adaptive_body<3, 2, NT, GammaPolicy<R>, CS>(pol, njobs, job_counter, cfg, scratch, slot_bytes);

@@ -81,6 +81,46 @@ constexpr I64Tables make_tables() {
 }
 }  // namespace i64detail
 
+// sin(pi (2 k + 1) / 256), Q64
+#if defined(__CUDACC__)
+static __device__ constexpr uint64_t d_i64sin[64] = {
+    0x03243a3f9bd8f08dull, 0x096c32baca2ae68bull, 0x0fb2b73cfc106ff7ull, 0x15f6d00a9aa418c1ull,
+    0x1c3785c79ec2d4f6ull, 0x2273e19db5eaed57ull, 0x28aaed62527cb3b6ull, 0x2edbb3bca17e628full,
+    0x3505404b6008a13cull, 0x3b269fca8a8622bbull, 0x413ee038dff6b7fdull, 0x474d10fd336cf747ull,
+    0x4d50430b860546c3ull, 0x53478909e39da892ull, 0x5931f774fc9f1844ull, 0x5f0ea4c477339c06ull,
+    0x64dca98ef24f5cb4ull, 0x6a9b20adb4ff262aull, 0x70492760047b9a7full, 0x75e5dd6e1b8e2555ull,
+    0x7b70654bbde35623ull, 0x80e7e43a61f5b6cbull, 0x864b826aec4c74e6ull, 0x8b9a6b1ef6da4502ull,
+    0x90d3ccc99f5ac58bull, 0x95f6d92fd79f4fbbull, 0x9b02c58832cf95c0ull, 0x9ff6ca9a2ab6a26dull,
+    0xa4d224dcd849c5b0ull, 0xa99414951aacae5full, 0xae3bddf3280c620dull, 0xb2c8c92f83c1eb88ull,
+    0xb73a22a755457448ull, 0xbb8f3af81b93095dull, 0xbfc7671ab8bb84c7ull, 0xc3e2007dd175f5a5ull,
+    0xc7de651f7ca06749ull, 0xcbbbf7a63eba0dd5ull, 0xcf7a1f794d7ca1b2ull, 0xd31848d817d70e17ull,
+    0xd695e4f10ea88570ull, 0xd9f269f7aab88c29ull, 0xdd2d5339ac8692fdull, 0xe046213392aa486cull,
+    0xe33c59a4439cd8ecull, 0xe60f879fe7e2e1e5ull, 0xe8bf3ba1f1aedfbcull, 0xeb4b0b9e4f345617ull,
+    0xedb29311c504d652ull, 0xeff573116df1555dull, 0xf21352595e0bf351ull, 0xf40bdd5a6688662full,
+    0xf5dec646f85ba1c7ull, 0xf78bc51f239e12c6ull, 0xf91297bbb1d6cdbeull, 0xfa7301d859796671ull,
+    0xfbaccd1d0903bb0aull, 0xfcbfc926484cd43bull, 0xfdabcb8caeba091cull, 0xfe70afeb6d33d6a2ull,
+    0xff0e57e5ead848d1ull, 0xff84ab2c738d6a03ull, 0xffd3977ff7bae4e9ull, 0xfffb10b4dc96dabcull,
+};
+#endif
+static constexpr uint64_t h_i64sin[64] = {
+    0x03243a3f9bd8f08dull, 0x096c32baca2ae68bull, 0x0fb2b73cfc106ff7ull, 0x15f6d00a9aa418c1ull,
+    0x1c3785c79ec2d4f6ull, 0x2273e19db5eaed57ull, 0x28aaed62527cb3b6ull, 0x2edbb3bca17e628full,
+    0x3505404b6008a13cull, 0x3b269fca8a8622bbull, 0x413ee038dff6b7fdull, 0x474d10fd336cf747ull,
+    0x4d50430b860546c3ull, 0x53478909e39da892ull, 0x5931f774fc9f1844ull, 0x5f0ea4c477339c06ull,
+    0x64dca98ef24f5cb4ull, 0x6a9b20adb4ff262aull, 0x70492760047b9a7full, 0x75e5dd6e1b8e2555ull,
+    0x7b70654bbde35623ull, 0x80e7e43a61f5b6cbull, 0x864b826aec4c74e6ull, 0x8b9a6b1ef6da4502ull,
+    0x90d3ccc99f5ac58bull, 0x95f6d92fd79f4fbbull, 0x9b02c58832cf95c0ull, 0x9ff6ca9a2ab6a26dull,
+    0xa4d224dcd849c5b0ull, 0xa99414951aacae5full, 0xae3bddf3280c620dull, 0xb2c8c92f83c1eb88ull,
+    0xb73a22a755457448ull, 0xbb8f3af81b93095dull, 0xbfc7671ab8bb84c7ull, 0xc3e2007dd175f5a5ull,
+    0xc7de651f7ca06749ull, 0xcbbbf7a63eba0dd5ull, 0xcf7a1f794d7ca1b2ull, 0xd31848d817d70e17ull,
+    0xd695e4f10ea88570ull, 0xd9f269f7aab88c29ull, 0xdd2d5339ac8692fdull, 0xe046213392aa486cull,
+    0xe33c59a4439cd8ecull, 0xe60f879fe7e2e1e5ull, 0xe8bf3ba1f1aedfbcull, 0xeb4b0b9e4f345617ull,
+    0xedb29311c504d652ull, 0xeff573116df1555dull, 0xf21352595e0bf351ull, 0xf40bdd5a6688662full,
+    0xf5dec646f85ba1c7ull, 0xf78bc51f239e12c6ull, 0xf91297bbb1d6cdbeull, 0xfa7301d859796671ull,
+    0xfbaccd1d0903bb0aull, 0xfcbfc926484cd43bull, 0xfdabcb8caeba091cull, 0xfe70afeb6d33d6a2ull,
+    0xff0e57e5ead848d1ull, 0xff84ab2c738d6a03ull, 0xffd3977ff7bae4e9ull, 0xfffb10b4dc96dabcull,
+};
+
 #if defined(__CUDACC__)
 static __device__ constexpr I64Tables d_i64tab = i64detail::make_tables();
 #endif
@@ -234,6 +274,34 @@ TP_HD int64_t i64_fix(double x) {
   return llrint(ldexp(x, B));
 #endif
 }
+
+// ---- sine and cosine ---------------------------------------------------------------
+// of x in [0, 8), Q62 signed, within 2^-60 absolute: the quarter turn's 64
+// cells by table, sin and cos of the distance d to a cell's centre
+// (|d| < pi/256) by their series to d^7 and d^6
+TP_HD void i64_sincos(double x, const uint64_t* __restrict__ tab, int64_t& sn, int64_t& cs) {
+  constexpr uint64_t INV_2PI = 0x28be60db9391054aull, PI_128 = 0x06487ed5110b4612ull;  // Q64
+  constexpr uint64_t R6 = 0x2aaaaaaaaaaaaaabull, R24 = 0x0aaaaaaaaaaaaaabull, R120 = 0x0222222222222222ull;
+  const uint64_t xf = (uint64_t)i64_fix<60>(x);
+  const uint64_t u = (i64_mulhi_exact(xf, INV_2PI) << 4) | ((xf * INV_2PI) >> 60);  // turns, Q64
+  const uint32_t quad = (uint32_t)(u >> 62), k = (uint32_t)(u >> 56) & 63u;
+  const int64_t r = (int64_t)((u << 8) ^ (1ull << 63));  // place in the cell minus 1/2, Q64
+  const uint64_t d = i64_mulhi((uint64_t)(r < 0 ? -r : r), PI_128 << 1) >> 1;  // (pi/2) / 64 of it
+  const uint64_t d2 = i64_mulhi(d, d);
+  const uint64_t h = (d2 >> 1) - i64_mulhi(d2, i64_mulhi(d2, R24 - (uint64_t)(((d2 >> 32) * 5965232u))));       // 1 - cos: 2^32 / 720
+  const uint64_t s = d - i64_mulhi(d, i64_mulhi(d2, R6 - i64_mulhi(d2, R120 - (uint64_t)((d2 >> 32) * 852176u))));  // sin: 2^32 / 5040
+  const uint64_t S = tab[k], C = tab[63 - k];
+  const int64_t Sh = (int64_t)(i64_mulhi(S, h) >> 2), Ch = (int64_t)(i64_mulhi(C, h) >> 2);
+  int64_t Cs = (int64_t)(i64_mulhi(C, s) >> 2), Ss = (int64_t)(i64_mulhi(S, s) >> 2);
+  if (r < 0) Cs = -Cs, Ss = -Ss;
+  const int64_t sv = (int64_t)(S >> 2) - Sh + Cs, cv = (int64_t)(C >> 2) - Ch - Ss;
+  // quarter turns: (s, c) -> (c, -s)
+  const int64_t a = (quad & 1) ? cv : sv, b = (quad & 1) ? sv : cv;
+  sn = (quad & 2) ? -a : a;
+  cs = ((quad + 1) & 2) ? -b : b;
+}
+// Q62 to double
+TP_HD double i64_q62(int64_t q) { return (double)q * 0x1p-62; }
 
 // ---- log2 -----------------------------------------------------------------------
 // log2 of a normalised mantissa m in [1, 2) (Q63): -log2 c + log2(1 + t) with
