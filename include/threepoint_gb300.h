@@ -267,9 +267,8 @@ int tp_gamma_batch(tp_ctx* ctx, int cosmo_index, const double* x, int n, int com
  * pixels over a square field of side fieldsize, the n_theta aperture radii
  * (fieldsize and thetas in the same unit, arcmin in the reference) and the
  * filter (polynomial != 0: Schneider's polynomial filter, else the
- * exponential one); it keeps on the device the Fourier transforms of the filter
- * grids of every aperture, so only the field's own transforms are done per
- * field. precision TP_FP64 does the transforms and Fourier products in FP64
+ * exponential one); it keeps on the device the filters' Fourier transforms of
+ * every aperture, so only the field's own transforms are done per field. precision TP_FP64 does the transforms and Fourier products in FP64
  * (the reference's numpy precision); TP_FP32 does them in FP32 (gridding, maps
  * and the <Map^3> sums stay FP64). Needs cuFFT at run time (loaded with
  * dlopen; TP_ERR_STATE if absent). */
@@ -279,7 +278,8 @@ int tp_apm_create(tp_ctx* ctx, int npix, double fieldsize, const double* thetas,
 /* A tp_apm's calls need its context; destroying it does not (it may come
  * after tp_ctx_destroy). */
 int tp_apm_destroy(tp_apm* apm);
-/* FFT grid side F >= 2 npix - 1 of the zero-padded convolutions */
+/* FFT grid side F of the zero-padded convolutions: at least 1.5 npix (the
+ * wrap-around stays outside the window that is kept), 2 npix - 1 with TP_FP32 */
 int tp_apm_fft_size(const tp_apm* apm);
 
 /* normalize_shear(Xs, Ys, shears, CIC=True, normalize=False) (:288-372):

@@ -106,6 +106,26 @@ def test_gpu_matches_oracle_other_sizes():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("n", [8, 9, 10, 63, 64, 101])
+def test_gpu_padding_edges(n, poly):
+    """Even and odd grids at and beside powers of two: the wrap-around of the
+    1.5 npix transforms must stay outside the window, and the separable filter
+    spectra must be the grids' (a wide aperture reaches across the grid).
+    Rounding of transforms of <= 150^2 values: below 1e-12 of the largest."""
+    tp, G = _gpu()
+    rng = np.random.default_rng(n)
+    fs, th = 20.0, 6.0
+    grid = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    w = rng.uniform(0.5, 1.5, (n, n))
+    with tp.Context(0) as ctx:
+        ac = G.aperture_mass_computer(n, th, fs, use_polynomial_filter=poly, ctx=ctx)
+        m, xm = ac.Map_fft(grid, norm=w, return_mcross=True)
+        rm, rx = A.map_weighted(grid, w, A.q_grid(n, fs, th, poly), return_cross=True)
+        assert rel(m, rm) < 1e-11 and rel(xm, rx) < 1e-11
+
+
+@pytest.mark.gpu
 def test_gpu_rejects_unsupported_options():
     tp, G = _gpu()
     with tp.Context(0) as ctx:

@@ -7,13 +7,21 @@
 // grid and normalize_weighted :199-286, norm_fft :283-286, normalize_shear
 // with CIC :288-372) and extract_Map3 / extract_Map3_of_field (:375-531).
 //
-// Design: one tp_apm object per (grid size, field size, apertures, filter)
-// keeps on the device the FFTs of the three filter grids of every aperture
-// (Re Q, Im Q and |Q| zero-padded to F x F, F >= 2 npix - 1), computed once,
-// so a field costs three forward transforms (the shear grid's real and
+// Design: a field costs three forward transforms (the shear grid's real and
 // imaginary parts and the weight grid) and two inverse ones per aperture
 // (numerator Im(g) * Im(Q) - Re(g) * Re(Q) and denominator w * |Q| multiplied
-// in Fourier space by one fused kernel). The 2-D FFTs are cuFFT's (loaded at
+// in Fourier space by one fused kernel). The filters of one (grid size, field
+// size, apertures, filter) are prepared once in a tp_apm. The exponential
+// filter's grids are sums of products of 1-D functions (Re Q, Im Q and |Q| are
+// (zr^2 - zi^2), -2 zr zi and (zr^2 + zi^2) times a Gaussian in zr and one in
+// zi), so in FP64 its spectra are products of three 1-D transforms formed where
+// they are used; the polynomial filter and the FP32 form keep the 2-D
+// transforms of the three zero-padded grids on the device. FP64 grids are
+// padded to F >= 1.5 npix: the wrap-around of a circular convolution of that
+// size stays outside the 'same' window that is kept (the FP32 form pads to
+// F >= 2 npix - 1). With both, <Map^3> of a 4096^2 field and four apertures from
+// its catalogue takes 11 transforms of 6144^2 instead of 23 of 8192^2, which
+// the FP64 pipe bounds: 213 -> 74 ms, plan included. The 2-D FFTs are cuFFT's (loaded at
 // run time with dlopen so that the rest of the library does not depend on
 // it), in FP64 (TP_FP64, the reference's numpy precision) or FP32 (TP_FP32:
 // transforms, filter spectra and Fourier products in FP32; gridding, maps and
@@ -210,6 +218,97 @@ __global__ void k_apm_pad(const double* __restrict__ src, int npix, int F, T* ds
   dst[(size_t)i * F + j] = (T)src[t];
 }
 
+// 1-D transforms of the exponential filter: with Q = C z^2 exp(-a z^2),
+// E_m(k) = sum_i z_i^m exp(-a z_i^2) exp(-2 pi I k i / F), z_i = i - npix / 2,
+// m = 0, 1, 2, k = 0 .. F/2 (E_m(F - k) is the conjugate). One thread a k,
+// blockIdx.y the aperture; the weights of a tile of i in shared memory, the
+// F-th roots of unity from a table. Direct sums, a tile at a time (so that the
+// rounding grows with the square roots of tile and tiles): 6 FP64 operations a
+// term, 0.6 ms for four apertures at F = 6144.
+constexpr int DFT_NT = 64, DFT_TILE = 64;
+__global__ void __launch_bounds__(DFT_NT) k_apm_dft1(int npix, int F, const double* __restrict__ a, const double2* __restrict__ tw, double2* E) {
+  __shared__ double w[3][DFT_TILE];
+  const int nk = F / 2 + 1, k = blockIdx.x * DFT_NT + threadIdx.x;
+  const double at = a[blockIdx.y];
+  double2 s[3] = {{0, 0}, {0, 0}, {0, 0}};
+  int t = 0;  // k i mod F
+  for (int i0 = 0; i0 < npix; i0 += DFT_TILE) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < DFT_TILE; i += DFT_NT) {
+      const double z = i0 + i - npix / 2.0, e = i0 + i < npix ? exp(-at * z * z) : 0.0;
+      w[0][i] = e;
+      w[1][i] = z * e;
+      w[2][i] = z * z * e;
+    }
+    __syncthreads();
+    if (k < nk) {
+      double2 p[3] = {{0, 0}, {0, 0}, {0, 0}};
+      for (int i = 0; i < DFT_TILE; ++i) {
+        const double2 u = tw[t];
+        t += k;
+        t = t >= F ? t - F : t;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          p[m].x = fma(w[m][i], u.x, p[m].x);
+          p[m].y = fma(w[m][i], u.y, p[m].y);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        s[m].x += p[m].x;
+        s[m].y += p[m].y;
+      }
+    }
+  }
+  if (k < nk)
+    for (int m = 0; m < 3; ++m) E[((size_t)blockIdx.y * 3 + m) * nk + k] = s[m];
+}
+
+__global__ void k_apm_roots(int F, double2* tw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= F) return;
+  double sn, cs;
+  sincospi(-2.0 * i / F, &sn, &cs);
+  tw[i] = make_double2(cs, sn);
+}
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// k_apm_spectra with the exponential filter's spectra from its 1-D transforms:
+// Re Q = C (E2 E0 - E0 E2), Im Q = -2 C E1 E1, |Q| = C (E2 E0 + E0 E2), first
+// factor the row frequency (blockIdx.x), second the column frequency. ~36 FP64
+// operations an entry (the FP64 pipe bounds it, as it does the transforms).
+__global__ void k_apm_spectra_sep(const double2* __restrict__ Yr, const double2* __restrict__ Yi,
+                                  const double2* __restrict__ W, const double2* __restrict__ E, double C, int F,
+                                  double2* num, double2* den, double2* cross) {
+  const int nk = F / 2 + 1, kx = blockIdx.x, ky = blockIdx.y * blockDim.x + threadIdx.x;
+  if (ky >= nk) return;
+  const int kr = kx < nk ? kx : F - kx;
+  double2 x[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    x[m] = E[(size_t)m * nk + kr];
+    if (kx != kr) x[m].y = -x[m].y;
+    x[m].x *= C;
+    x[m].y *= C;
+  }
+  const double2 y0 = E[ky], y1 = E[(size_t)nk + ky], y2 = E[(size_t)2 * nk + ky];
+  const double2 p = cmul(x[1], y1), s = cmul(x[2], y0), t = cmul(x[0], y2);
+  const double2 qr = make_double2(s.x - t.x, s.y - t.y), qi = make_double2(-2 * p.x, -2 * p.y),
+                qa = make_double2(s.x + t.x, s.y + t.y);
+  const size_t o = (size_t)kx * nk + ky;
+  const double2 yr = Yr[o], yi = Yi[o];
+  const double2 u = cmul(yi, qi), v = cmul(yr, qr);
+  num[o] = make_double2(u.x - v.x, u.y - v.y);
+  den[o] = cmul(W[o], qa);
+  if (cross) {
+    const double2 c = cmul(yr, qi), d = cmul(yi, qr);
+    cross[o] = make_double2(-(c.x + d.x), -(c.y + d.y));
+  }
+}
+
 // Fourier-space products of one aperture: num = Im(g) Im(Q) - Re(g) Re(Q),
 // den = w |Q| (Map_fft :211-236 with norm_fft :283-286), cross (optional) =
 // -(Re(g) Im(Q) + Im(g) Re(Q)) (return_mcross :246-255)
@@ -372,7 +471,9 @@ struct tp_apm {
   // transform buffers, in the precision's real / complex type
   char* pad = nullptr;                              // [3][F][F] padded real grids
   char* spec = nullptr;                             // [3][F][F/2+1]: Re g, Im g, w
-  char* qspec = nullptr;                            // [n_theta][3][F][F/2+1]: Re Q, Im Q, |Q|
+  bool sep = false;                                 // filter spectra from the 1-D transforms
+  double2* e1d = nullptr;                           // [n_theta][3][F/2+1] (sep)
+  char* qspec = nullptr;                            // [n_theta][3][F][F/2+1]: Re Q, Im Q, |Q| (not sep)
   char* work = nullptr;                             // [3][F][F/2+1]: num, den, cross
   double* maps = nullptr;                           // [n_theta][npix][npix]
   double* mcross = nullptr;                         // [n_theta][npix][npix] (allocated on demand)
@@ -451,10 +552,18 @@ int apm_maps_t(tp_apm* a, bool want_cross) {
   }
   const C* Y = (const C*)a->spec;
   for (int t = 0; t < a->n_theta; ++t) {
-    const C* Q = (const C*)a->Cx(a->qspec, 3 * (size_t)t);
     C* W = (C*)a->work;
     const long nc = (long)a->ncplx;
-    k_apm_spectra<C><<<blocks_for(nc, 256), 256, 0, s>>>(Y, Y + nc, Y + 2 * nc, Q, Q + nc, Q + 2 * nc, nc, W, W + nc,
+    const C* Q = a->sep ? nullptr : (const C*)a->Cx(a->qspec, 3 * (size_t)t);
+    if constexpr (sizeof(T) == 8) {
+      if (a->sep) {
+        const double b = a->fieldsize / ((double)n * a->thetas[t]), c = b * b / (4 * PI * a->thetas[t] * a->thetas[t]);
+        k_apm_spectra_sep<<<dim3(F, blocks_for(F / 2 + 1, 256)), 256, 0, s>>>(
+            Y, Y + nc, Y + 2 * nc, a->e1d + (size_t)t * 3 * (F / 2 + 1), c, F, W, W + nc, want_cross ? W + 2 * nc : nullptr);
+      }
+    }
+    if (!a->sep)
+      k_apm_spectra<C><<<blocks_for(nc, 256), 256, 0, s>>>(Y, Y + nc, Y + 2 * nc, Q, Q + nc, Q + 2 * nc, nc, W, W + nc,
                                                         want_cross ? W + 2 * nc : nullptr);
     e = cudaGetLastError();
     if (e != cudaSuccess) return apm_cuda(a, e, "apm spectra");
@@ -474,6 +583,27 @@ int apm_maps_t(tp_apm* a, bool want_cross) {
 
 int apm_maps_device(tp_apm* a, bool want_cross) {
   return a->precision == TP_FP64 ? apm_maps_t<double, double2>(a, want_cross) : apm_maps_t<float, float2>(a, want_cross);
+}
+
+// the exponential filter's 1-D transforms of every aperture
+int apm_filters_1d(tp_apm* a) {
+  cudaStream_t s = a->ctx->stream;
+  std::vector<double> at(a->n_theta);
+  for (int t = 0; t < a->n_theta; ++t) {
+    const double b = a->fieldsize / ((double)a->npix * a->thetas[t]);
+    at[t] = 0.5 * b * b;
+  }
+  // roots of unity and exponents in the transform buffer
+  double2* tw = (double2*)a->work;
+  double* da = (double*)(tw + a->F);
+  cudaError_t e = cudaMemcpyAsync(da, at.data(), sizeof(double) * a->n_theta, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) {
+    k_apm_roots<<<blocks_for(a->F, 256), 256, 0, s>>>(a->F, tw);
+    k_apm_dft1<<<dim3(blocks_for(a->F / 2 + 1, DFT_NT), a->n_theta), DFT_NT, 0, s>>>(a->npix, a->F, da, tw, a->e1d);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // at leaves scope
+  return apm_cuda(a, e, "apm 1-D filters");
 }
 
 // the Fourier transforms of the Q filter grids of every aperture
@@ -578,7 +708,12 @@ extern "C" int tp_apm_create(tp_ctx* ctx, int npix, double fieldsize, const doub
   a->rsz = precision == TP_FP64 ? sizeof(double) : sizeof(float);
   a->csz = precision == TP_FP64 ? sizeof(double2) : sizeof(float2);
   a->thetas.assign(thetas, thetas + n_theta);
-  a->F = fft_size(2 * npix - 1);
+  a->sep = precision == TP_FP64 && !polynomial;
+  // 'same' window [off, off + npix) of a linear convolution of 2 npix - 1: index
+  // k wraps onto k +- F, which must be outside the window or the convolution
+  const int off = (npix - 1) / 2;
+  // (an even size: the three grids then start on complex-value boundaries)
+  a->F = precision == TP_FP64 ? 2 * fft_size((std::max(2 * npix - 1 - off, off + npix) + 1) / 2) : fft_size(2 * npix - 1);
   a->nreal = (size_t)a->F * a->F;
   a->ncplx = (size_t)a->F * (a->F / 2 + 1);
   const size_t npx = (size_t)npix * npix;
@@ -597,7 +732,10 @@ extern "C" int tp_apm_create(tp_ctx* ctx, int npix, double fieldsize, const doub
   M(&a->g_w, sizeof(double) * npx);
   M(&a->pad, a->rsz * 3 * a->nreal);
   M(&a->spec, a->csz * 3 * a->ncplx);
-  M(&a->qspec, a->csz * 3 * a->ncplx * n_theta);
+  if (a->sep)
+    M(&a->e1d, sizeof(double2) * 3 * (a->F / 2 + 1) * n_theta);
+  else
+    M(&a->qspec, a->csz * 3 * a->ncplx * n_theta);
   M(&a->work, a->csz * 3 * a->ncplx);
   M(&a->maps, sizeof(double) * npx * n_theta);
   M(&a->sums, sizeof(double) * nt);
@@ -633,7 +771,7 @@ extern "C" int tp_apm_create(tp_ctx* ctx, int npix, double fieldsize, const doub
     e = cudaMemcpyAsync(a->cut_same, a->h_cut_same.data(), sizeof(int) * n_theta, cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return fail(tp_cuda(ctx, e, "apm upload"));
   // the filter spectra of every aperture, computed once
-  const int st = f64 ? apm_filters_t<double>(a) : apm_filters_t<float>(a);
+  const int st = a->sep ? apm_filters_1d(a) : f64 ? apm_filters_t<double>(a) : apm_filters_t<float>(a);
   if (st) return fail(st);
   *out = a;
   return TP_OK;
@@ -647,7 +785,7 @@ extern "C" int tp_apm_destroy(tp_apm* a) {
   if (a->have_fwd) api.destroy(a->fwd);
   if (a->have_inv) api.destroy(a->inv);
   for (void* p : {(void*)a->edges, (void*)a->g_re, (void*)a->g_im, (void*)a->g_w, (void*)a->pad, (void*)a->spec,
-                  (void*)a->qspec, (void*)a->work, (void*)a->maps, (void*)a->mcross, (void*)a->sums, (void*)a->counts,
+                  (void*)a->qspec, (void*)a->e1d, (void*)a->work, (void*)a->maps, (void*)a->mcross, (void*)a->sums, (void*)a->counts,
                   (void*)a->outv, (void*)a->cut, (void*)a->cut_same, (void*)a->uspec})
     if (p) cudaFree(p);
   delete a;
