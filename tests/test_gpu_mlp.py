@@ -93,3 +93,42 @@ def test_training_reduces_loss(net):
     net.sync()
     l1, _ = net.gradients(x, t)
     assert l1 < 0.05 * l0, (l0, l1)
+
+
+# both GEMM forms at their edges: one and four slabs of the resident form with
+# fewer and more row tiles than SMs, slab rings shorter and longer than the ring,
+# column counts whose halves differ. BF16 products are exact in FP32, so the
+# error is that of K roundings of sums: K 2^-24 of the largest partial sum
+@pytest.mark.parametrize("M_,N,K", [(128, 32, 64), (128 * 153, 96, 64), (128 * 310, 256, 256), (256, 160, 192),
+                                    (128, 256, 320), (384, 96, 448), (256, 224, 2048)])
+def test_gemm_forms_at_their_edges(net, M_, N, K):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(M_ + N + K)
+    A = torch.randn(M_, K, generator=g, device="cuda").to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    Cm = torch.full((M_, N), float("nan"), dtype=torch.float32, device="cuda")
+    net.gemm_device(A, B, Cm)
+    ref = A.double() @ B.double().T
+    bound = K * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T)
+    assert bool(((Cm.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 4096])
+def test_gradients_at_batch_edges(n):
+    """One row, rows beside a tile edge and a batch longer than a segment of the
+    bias sums, against the FP64 network with the same BF16 operands (relative to
+    each layer's largest gradient: two BF16 roundings of 2^-9 a layer)"""
+    import threepoint_gb300 as tp
+
+    ps, x, t = params_and_data(n, seed=n)
+    _, grads = M.loss_and_grads(ps, x, t, round_bf16=True)
+    m = tp.MLP(max_batch=4096)
+    try:
+        m.set_params(ps)
+        _, got = m.gradients(x, t)
+    finally:
+        m.close()
+    for (gW, gb), (rW, rb) in zip(got, grads):
+        assert np.abs(gW - rW).max() <= 3e-2 * np.abs(rW).max() + 1e-12
+        assert np.abs(gb - rb).max() <= 3e-2 * np.abs(rb).max() + 1e-12

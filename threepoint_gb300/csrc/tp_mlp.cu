@@ -2,16 +2,17 @@
 // multilayer perceptron 8 -> 256 -> 256 -> 256 -> 256 -> 1 (SiLU after the
 // hidden layers) trained and evaluated with BF16 operands and FP32
 // accumulation. Every layer is one GEMM C = A B^T (A [M x K], B [N x K], both
-// BF16 with K contiguous) on tcgen05: one CTA computes a 128 x N tile
-// (N <= 256) into tensor memory, with K in 64-wide slabs staged in shared
-// memory in the 128-byte-swizzled K-major layout (two buffers: the next slab
-// loads while the tensor core consumes the current one); one thread issues
-// the MMAs and commits them to the buffer's mbarrier; the four warps read the
-// accumulator back (tcgen05.ld) and apply the layer's epilogue (bias, SiLU or
-// its derivative, BF16 row-major and transposed copies for the next layer and
-// the weight gradients, the last layer's dot product). Weight gradients are
-// the same GEMM over the batch (K = batch) split into K slices whose FP32
-// partials a second kernel sums in a fixed order.
+// BF16 with K contiguous) on tcgen05: a CTA computes 128 x N tiles (N <= 256)
+// into tensor memory from 64-wide K slabs staged in shared memory in the
+// 128-byte-swizzled K-major layout by asynchronous copies; one thread issues
+// the MMAs and commits them to an mbarrier; sixteen warps read the accumulator
+// back (tcgen05.ld) and apply the layer's epilogue (bias, SiLU or its
+// derivative, BF16 row-major and transposed copies for the next layer and the
+// weight gradients, the last layer's dot product). The layers (K <= 256) keep
+// the whole weight matrix in shared memory and run persistently over the row
+// tiles, the next tile's rows loading during the epilogue; weight gradients
+// are a GEMM over the batch (K = batch) with a ring of four slabs, split into
+// K slices whose FP32 partials a second kernel sums in a fixed order.
 //
 // Every mbarrier wait has an iteration limit: on expiry the kernel raises an
 // error flag, waits (bounded) for its committed MMAs, frees its tensor memory
@@ -32,7 +33,7 @@ namespace tp {
 constexpr int MLP_IN = 8;       // features
 constexpr int MLP_IN_PAD = 64;  // first layer's K (one 64-wide slab, zero padded)
 constexpr int MLP_W = 256;      // hidden width
-constexpr int GEMM_NT = 128;    // threads of the GEMM CTA (4 warps = 128 TMEM lanes)
+constexpr int GEMM_NT = 512;    // threads of a GEMM CTA: four warps per 32 TMEM lanes
 constexpr int GEMM_BM = 128;    // rows per CTA tile
 constexpr int GEMM_BK = 64;     // K per slab (one 128-byte swizzle atom of BF16)
 constexpr int MBAR_SPIN = 1 << 22;
@@ -131,164 +132,305 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v) {
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tc_st32(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+      "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+      "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+      "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
+      "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
+      "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
+      "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
+      "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// eight words, a whole 32-byte sector, a lane
+__device__ __forceinline__ void st8(void* p, const uint32_t* r) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void st8(float* p, const float* v) {
+  uint32_t r[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) r[i] = __float_as_uint(v[i]);
+  st8((void*)p, r);
+}
+__device__ __forceinline__ void ld8(float* v, const float* p) {
+  uint32_t r[8];
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(p)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 __device__ __forceinline__ float silu_grad_f(float z) {
   const float s = 1.f / (1.f + __expf(-z));
   return s * (1.f + z * (1.f - s));
 }
 
-// stage one 64-wide K slab of `rows` rows (K-major, 16-byte chunks) into the
-// swizzled layout
-__device__ __forceinline__ void load_slab(char* dst, const __nv_bfloat16* src, int ld, int rows, int k0) {
+// copy one 64-wide K slab of `rows` rows (K-major, 16-byte chunks) into the
+// swizzled layout, asynchronously
+__device__ __forceinline__ void load_slab(uint32_t dst, const __nv_bfloat16* src, int ld, int rows, int k0) {
   const int chunks = rows * 8;
   for (int q = threadIdx.x; q < chunks; q += GEMM_NT) {
     const int r = q >> 3, c = q & 7;
-    const uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)r * ld + k0 + 8 * c);
-    *reinterpret_cast<uint4*>(dst + r * 128 + ((c ^ (r & 7)) << 4)) = v;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + r * 128 + ((c ^ (r & 7)) << 4)),
+                 "l"(src + (size_t)r * ld + k0 + 8 * c)
+                 : "memory");
+  }
+}
+__device__ __forceinline__ void load_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void load_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// four MMAs of one 64-wide slab (K order: slabs ascending, 16 at a time)
+__device__ __forceinline__ void mma_slab(uint32_t tmem, uint32_t a0, uint32_t b0, uint32_t idesc, bool first) {
+#pragma unroll
+  for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+    tc_mma(tmem, smem_desc_sw128(a0 + 32 * kk), smem_desc_sw128(b0 + 32 * kk), idesc, !first || kk != 0);
+}
+
+constexpr size_t GEMM_SLAB_A = (size_t)GEMM_BM * GEMM_BK * 2;
+constexpr size_t GEMM_SLAB_B = (size_t)MLP_W * GEMM_BK * 2;
+constexpr int GEMM_KMAX = 256, GEMM_STAGES = 4;             // k_gemm_rows' K; k_gemm_ring's slabs in flight
+constexpr size_t GEMM_SMEM = 1024 + GEMM_STAGES * (GEMM_SLAB_A + GEMM_SLAB_B) + 64;
+static_assert(GEMM_STAGES * GEMM_BK >= GEMM_KMAX, "k_gemm_rows holds every slab of A and B");
+
+// The epilogue of the 128 x N tile at row m0 in tensor memory: warp w takes
+// the 32 rows of lanes 32 (w % 4) and every fourth 32-column chunk from w / 4
+// on, a row a lane. Row-major operands and results move a 32-byte sector a
+// lane and instruction: whole sectors without a pass through shared memory, so
+// that sixteen warps fit beside the slabs.
+__device__ __forceinline__ void gemm_epilogue(const GemmArgs& g, uint32_t tmem, int m0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = warp >> 2;
+  const int row = m0 + quad * 32 + lane;
+  const uint32_t tw = tmem + ((uint32_t)(quad * 32) << 16);
+  const int f = g.flags, nch = g.N / 32;
+  for (int c = part; c < nch; c += GEMM_NT / 128) {
+    const int c0 = 32 * c;
+    float v[32], zin[32];
+    if (f & EPI_DSILU) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ld8(zin + 8 * q, g.zin + (size_t)row * g.ldzin + c0 + 8 * q);
+    }
+    tc_ld32(tw + (uint32_t)c0, v);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float z[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int j = 8 * q + i;
+        z[i] = v[j];
+        if (f & EPI_BIAS) z[i] += g.bias[c0 + j];
+        if (f & EPI_DSILU) z[i] *= silu_grad_f(zin[j]);
+        v[j] = (f & EPI_SILU) ? silu_f(z[i]) : z[i];
+      }
+      if (f & EPI_STORE_Z) st8(g.zout + (size_t)row * g.ldz + c0 + 8 * q, z);
+    }
+    if (f & EPI_STORE_HT) {
+      // two rows (this lane's and its neighbour's) of one column a lane
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? v[j] : v[j + 1], 1);
+        const __nv_bfloat162 p = (lane & 1) ? __floats2bfloat162_rn(other, v[j + 1]) : __floats2bfloat162_rn(v[j], other);
+        *reinterpret_cast<__nv_bfloat162*>(g.ht + (size_t)(c0 + j + (lane & 1)) * g.ldht + (row & ~1)) = p;
+      }
+    }
+    if (f & EPI_STORE_F32) {
+      float* o = g.out + (size_t)blockIdx.y * g.split_stride + (size_t)row * g.ldo + c0;
+      if (((size_t)g.out & 31) == 0 && g.ldo % 8 == 0) {  // (split_stride is a multiple of 8)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) st8(o + 8 * q, v + 8 * q);
+      } else {  // a caller's matrix of any alignment
+#pragma unroll
+        for (int j = 0; j < 32; ++j) o[j] = v[j];
+      }
+    }
+    if (f & EPI_STORE_H) {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const __nv_bfloat162 p = __floats2bfloat162_rn(v[16 * q + 2 * i], v[16 * q + 2 * i + 1]);
+          r[i] = *reinterpret_cast<const uint32_t*>(&p);
+        }
+        st8(g.h + (size_t)row * g.ldh + c0 + 16 * q, r);
+      }
+    }
+    if (f & EPI_DOT) tc_st32(tw + (uint32_t)c0, v);
+  }
+  if (f & EPI_DOT) {
+    // one chain over the columns of a row, from the results put back in tensor memory
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (part == 0) {
+      float dot = 0.f;
+      for (int c = 0; c < nch; ++c) {
+        float v[32];
+        tc_ld32(tw + (uint32_t)(32 * c), v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) dot = fmaf(v[j], g.w5[32 * c + j], dot);
+      }
+      g.y[row] = dot + *g.b5;
+    }
   }
 }
 
-// dynamic shared memory: 2 x (A slab 16 KB + B slab up to 32 KB), 1024-aligned
-constexpr size_t GEMM_SLAB_A = (size_t)GEMM_BM * GEMM_BK * 2;
-constexpr size_t GEMM_SLAB_B = (size_t)MLP_W * GEMM_BK * 2;
-constexpr size_t GEMM_SMEM = 1024 + 2 * (GEMM_SLAB_A + GEMM_SLAB_B) + 64;
-
-__global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_tc(GemmArgs g) {
-  extern __shared__ __align__(16) char smem_raw[];
-  // swizzled tiles need a 1024-byte aligned shared-memory address
-  char* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  char* sa[2] = {base, base + GEMM_SLAB_A};
-  char* sb[2] = {base + 2 * GEMM_SLAB_A, base + 2 * GEMM_SLAB_A + GEMM_SLAB_B};
-  uint64_t* bars = (uint64_t*)(base + 2 * (GEMM_SLAB_A + GEMM_SLAB_B));
-  uint32_t* s_tmem = (uint32_t*)(bars + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * GEMM_BM;
-  const int kper = g.K / g.kslices, kbeg = blockIdx.y * kper;
-  const int nslab = kper / GEMM_BK;
-  const int N = g.N;
-  const int ncols = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256;
-  const uint32_t bar0 = smem_u32(&bars[0]), bar1 = smem_u32(&bars[1]);
-
+// shared memory of a GEMM CTA: slabs (1024-byte aligned), barriers
+struct GemmSmem {
+  uint32_t a, b;  // slab s of A at a + s GEMM_SLAB_A, of B at b + s GEMM_SLAB_B
+  uint64_t* bars;
+  uint32_t* tmem;
+  __device__ __forceinline__ GemmSmem(char* raw) {
+    char* base = raw + ((1024u - (smem_u32(raw) & 1023u)) & 1023u);
+    a = smem_u32(base);
+    b = a + GEMM_STAGES * GEMM_SLAB_A;
+    bars = (uint64_t*)(base + GEMM_STAGES * (GEMM_SLAB_A + GEMM_SLAB_B));
+    tmem = (uint32_t*)(bars + GEMM_STAGES);
+  }
+};
+__device__ __forceinline__ int tmem_cols(int N) { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256; }
+__device__ __forceinline__ void gemm_begin(const GemmSmem& m, int N) {
   if (threadIdx.x == 0) {
-    mbar_init(bar0, 1);
-    mbar_init(bar1, 1);
+    for (int s = 0; s < GEMM_STAGES; ++s) mbar_init(smem_u32(&m.bars[s]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
-                 "r"(ncols)
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(m.tmem)),
+                 "r"(tmem_cols(N))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *s_tmem;
-  const uint32_t idesc = idesc_bf16_m128(N);
-  bool ok = true;
+}
+__device__ __forceinline__ void gemm_end(const GemmArgs& g, uint32_t tmem, bool ok) {
+  if (!ok && threadIdx.x == 0 && g.err) atomicOr(g.err, 1u);
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols(g.N)) : "memory");
+}
 
-  for (int s = 0; s < nslab && ok; ++s) {
-    const int b = s & 1;
-    if (s >= 2) ok = mbar_wait(b ? bar1 : bar0, ((s - 2) >> 1) & 1);  // buffer b free again
+// K <= GEMM_KMAX: B stays in shared memory, the CTA walks the row tiles
+// blockIdx.x, + gridDim.x, ...; the next tile's rows of A are copied while this
+// tile's epilogue runs. The epilogue's stores bound it (HBM: 167 MB for a
+// training layer of 65536 rows, 25 us): 177 -> 62 us for that layer with sixteen
+// warps on the accumulator, 100 us with eight and a shared-memory transpose,
+// against one tile a CTA whose loads, MMAs and epilogue wait for one another
+__global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_rows(GemmArgs g) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const GemmSmem m(smem_raw);
+  gemm_begin(m, g.N);
+  const uint32_t tmem = *m.tmem, bar = smem_u32(&m.bars[0]), idesc = idesc_bf16_m128(g.N);
+  const int nslab = g.K / GEMM_BK, ntile = g.M / GEMM_BM;
+  auto load_a = [&](int t) {
+    for (int s = 0; s < nslab; ++s)
+      load_slab(m.a + s * GEMM_SLAB_A, g.A + (size_t)t * GEMM_BM * g.lda, g.lda, GEMM_BM, s * GEMM_BK);
+    load_commit();
+  };
+  for (int s = 0; s < nslab; ++s) load_slab(m.b + s * GEMM_SLAB_B, g.B, g.ldb, g.N, s * GEMM_BK);
+  if ((int)blockIdx.x < ntile) load_a(blockIdx.x);
+  bool ok = true;
+  uint32_t parity = 0;
+  for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
+    load_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();  // the previous epilogue's accumulator reads
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      tc_fence_after();
+      for (int s = 0; s < nslab; ++s) mma_slab(tmem, m.a + s * GEMM_SLAB_A, m.b + s * GEMM_SLAB_B, idesc, s == 0);
+      tc_commit(bar);
+    }
+    ok = mbar_wait(bar, parity);
+    parity ^= 1;
     ok = __syncthreads_and(ok);
     if (!ok) break;
-    const int k0 = kbeg + s * GEMM_BK;
-    load_slab(sa[b], g.A + (size_t)m0 * g.lda, g.lda, GEMM_BM, k0);
-    load_slab(sb[b], g.B, g.ldb, N, k0);
+    tc_fence_after();
+    if (t + (int)gridDim.x < ntile) load_a(t + gridDim.x);
+    gemm_epilogue(g, tmem, t * GEMM_BM);
+  }
+  load_wait<0>();
+  gemm_end(g, tmem, ok);
+}
+
+// Any K: a ring of GEMM_STAGES slabs of A and B; blockIdx.x the row tile,
+// blockIdx.y the K slice. The copies of three slabs are in flight while the
+// tensor core works on the fourth (a 256 x 256 weight gradient over 65536 rows
+// in 64 slices: 222 -> 25 us, against two slabs and a wait after each load)
+__global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_ring(GemmArgs g) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const GemmSmem m(smem_raw);
+  gemm_begin(m, g.N);
+  const uint32_t tmem = *m.tmem, idesc = idesc_bf16_m128(g.N);
+  const int m0 = blockIdx.x * GEMM_BM, kper = g.K / g.kslices, kbeg = blockIdx.y * kper, nslab = kper / GEMM_BK;
+  auto load = [&](int s) {  // a group a slab, empty past the end
+    if (s < nslab) {
+      const int b = s % GEMM_STAGES;
+      load_slab(m.a + b * GEMM_SLAB_A, g.A + (size_t)m0 * g.lda, g.lda, GEMM_BM, kbeg + s * GEMM_BK);
+      load_slab(m.b + b * GEMM_SLAB_B, g.B, g.ldb, g.N, kbeg + s * GEMM_BK);
+    }
+    load_commit();
+  };
+  for (int s = 0; s < GEMM_STAGES - 1; ++s) load(s);
+  bool ok = true;
+  for (int s = 0; s < nslab; ++s) {
+    load_wait<GEMM_STAGES - 2>();  // slab s has landed
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (threadIdx.x == 0) {
       tc_fence_after();
-      const uint32_t a0 = smem_u32(sa[b]), b0 = smem_u32(sb[b]);
-#pragma unroll
-      for (int kk = 0; kk < GEMM_BK / 16; ++kk)
-        tc_mma(tmem, smem_desc_sw128(a0 + 32 * kk), smem_desc_sw128(b0 + 32 * kk), idesc, (s | kk) != 0);
-      tc_commit(b ? bar1 : bar0);
+      const int b = s % GEMM_STAGES;
+      mma_slab(tmem, m.a + b * GEMM_SLAB_A, m.b + b * GEMM_SLAB_B, idesc, s == 0);
+      tc_commit(smem_u32(&m.bars[b]));
     }
+    // slab s - 1's buffer is free once its MMAs are done: slab s + 3 goes there
+    if (s > 0) {
+      ok = mbar_wait(smem_u32(&m.bars[(s - 1) % GEMM_STAGES]), ((s - 1) / GEMM_STAGES) & 1);
+      ok = __syncthreads_and(ok);
+      if (!ok) break;
+    }
+    load(s + GEMM_STAGES - 1);
   }
-  // the last commit covers every MMA of the CTA
-  if (nslab > 0) {
-    const int last = nslab - 1;
-    const bool done = mbar_wait((last & 1) ? bar1 : bar0, (last >> 1) & 1);
-    ok = ok && done;
-  }
+  if (ok) ok = mbar_wait(smem_u32(&m.bars[(nslab - 1) % GEMM_STAGES]), ((nslab - 1) / GEMM_STAGES) & 1);
   ok = __syncthreads_and(ok);
+  load_wait<0>();
   tc_fence_after();
-
-  if (ok && nslab > 0) {
-    const int row0 = m0 + warp * 32;  // this warp's 32 rows; lane = row in the accumulator
-    const int row = row0 + lane;
-    const uint32_t tw = tmem + ((uint32_t)(warp * 32) << 16);
-    float dot = 0.f;
-    const int f = g.flags;
-    // Row-major operands and results go through a per-warp 32 x 33 shared
-    // tile (the slab buffers are free once the last MMA has completed), so
-    // that global loads and stores move whole rows (32 consecutive columns per
-    // instruction) instead of one element per lane and row.
-    float* tile = reinterpret_cast<float*>(sb[0]) + warp * 32 * 33;
-    for (int c0 = 0; c0 < N; c0 += 32) {
-      float v[32];
-      tc_ld32(tw + (uint32_t)c0, v);
-      float zin[32];
-      if (f & EPI_DSILU) {
-        for (int r = 0; r < 32; ++r) tile[r * 33 + lane] = g.zin[(size_t)(row0 + r) * g.ldzin + c0 + lane];
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) zin[j] = tile[lane * 33 + j];
-        __syncwarp();
-      }
-      float zv[32], hv[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int col = c0 + j;
-        float z = v[j];
-        if (f & EPI_BIAS) z += g.bias[col];
-        if (f & EPI_DSILU) z *= silu_grad_f(zin[j]);
-        zv[j] = z;
-        const float hval = (f & EPI_SILU) ? silu_f(z) : z;
-        hv[j] = hval;
-        if (f & EPI_STORE_HT) g.ht[(size_t)col * g.ldht + row] = __float2bfloat16_rn(hval);
-        if (f & EPI_DOT) dot = fmaf(hval, g.w5[col], dot);
-      }
-      if (f & EPI_STORE_Z) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = zv[j];
-        __syncwarp();
-        for (int r = 0; r < 32; ++r) g.zout[(size_t)(row0 + r) * g.ldz + c0 + lane] = tile[r * 33 + lane];
-        __syncwarp();
-      }
-      if (f & (EPI_STORE_F32 | EPI_STORE_H)) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = hv[j];
-        __syncwarp();
-        for (int r = 0; r < 32; ++r) {
-          const float x = tile[r * 33 + lane];
-          if (f & EPI_STORE_F32)
-            g.out[(size_t)blockIdx.y * g.split_stride + (size_t)(row0 + r) * g.ldo + c0 + lane] = x;
-          if (f & EPI_STORE_H) g.h[(size_t)(row0 + r) * g.ldh + c0 + lane] = __float2bfloat16_rn(x);
-        }
-        __syncwarp();
-      }
-    }
-    if (f & EPI_DOT) g.y[row] = dot + *g.b5;
-  }
-  if (!ok && threadIdx.x == 0 && g.err) atomicOr(g.err, 1u);
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+  if (ok) gemm_epilogue(g, tmem, m0);
+  gemm_end(g, tmem, ok);
 }
 
 // ---- element-wise and reduction kernels of the training step ---------------
 
-// features [n][8] (FP32) -> X [Mpad][64] and XT [64][Mpad] (BF16, zero padded)
+// features [n][8] (FP32) -> X [Mpad][64] and the first 8 rows of XT [64][Mpad]
+// (BF16, zero padded; the caller clears the other rows); one thread a row, so
+// that both are written in whole sectors
 __global__ void k_mlp_pack(const float* x, long n, int mpad, __nv_bfloat16* X, __nv_bfloat16* XT) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)mpad * MLP_IN_PAD) return;
-  const int r = (int)(i / MLP_IN_PAD), c = (int)(i % MLP_IN_PAD);
-  const float v = (r < n && c < MLP_IN) ? x[(size_t)r * MLP_IN + c] : 0.f;
-  X[i] = __float2bfloat16_rn(v);
-  XT[(size_t)c * mpad + r] = __float2bfloat16_rn(v);
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= mpad) return;
+  alignas(16) __nv_bfloat16 v[MLP_IN];
+#pragma unroll
+  for (int c = 0; c < MLP_IN; ++c) {
+    v[c] = __float2bfloat16_rn(r < n ? x[(size_t)r * MLP_IN + c] : 0.f);
+    XT[(size_t)c * mpad + r] = v[c];
+  }
+  uint4* o = reinterpret_cast<uint4*>(X + (size_t)r * MLP_IN_PAD);
+  o[0] = *reinterpret_cast<const uint4*>(v);
+#pragma unroll
+  for (int q = 1; q < MLP_IN_PAD / 8; ++q) o[q] = make_uint4(0, 0, 0, 0);
 }
 
 // dy = 2 (y - t) / n (0 on padding rows); per-block partial sums of (y - t)^2
@@ -313,21 +455,72 @@ __global__ void k_mlp_loss(const float* y, const float* t, long n, int mpad, flo
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// sum of nparts doubles in a fixed order (one thread)
+// sum of nparts doubles in a fixed order (one thread, from shared memory)
 __global__ void k_sum_fixed(const double* part, int nparts, long n, float* loss) {
-  if (threadIdx.x || blockIdx.x) return;
+  __shared__ double sp[1024];
   double s = 0;
-  for (int i = 0; i < nparts; ++i) s += part[i];
-  *loss = (float)(s / (double)n);
+  for (int i0 = 0; i0 < nparts; i0 += 1024) {
+    const int m = min(1024, nparts - i0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < m; i += blockDim.x) sp[i] = part[i0 + i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) s += sp[i];
+    }
+  }
+  if (threadIdx.x == 0) *loss = (float)(s / (double)n);
 }
 
-// dW5[j] = sum_b dy[b] h4[b][j], db5 = sum_b dy[b]: one warp per column j
-// (and one extra warp for db5), fixed summation order per lane then butterfly
-__global__ void k_mlp_last_grad(const float* dy, const float* h4, int mpad, float* gw5, float* gb5) {
+// dW5[j] = sum_b dy[b] h4[b][j], db5 = sum_b dy[b] in 32 chains (b mod 32)
+// whose sums a butterfly adds: one block a chain and 64 columns, a thread a
+// column, so that 128 blocks read whole row pieces. A chain is serial, so its
+// rows are copied ahead, three of four stages of 32 rows in flight (335 -> 34
+// us for 65536 rows, against one warp a column)
+constexpr int LG_COLS = 64, LG_ROWS = 32, LG_STAGES = 4;
+__global__ void __launch_bounds__(LG_COLS) k_mlp_last_grad(const float* dy, const float* h4, int mpad, float* part) {
+  __shared__ __align__(16) float sh[LG_STAGES][LG_ROWS][LG_COLS];
+  __shared__ float sd[LG_STAGES][LG_ROWS];
+  const int l = blockIdx.x, c0 = blockIdx.y * LG_COLS, tid = threadIdx.x;
+  const int nrow = mpad / 32, ns = (nrow + LG_ROWS - 1) / LG_ROWS;
+  auto load = [&](int k) {  // a group a stage, empty past the end
+    if (k < ns) {
+      const int b = k % LG_STAGES, n = min(LG_ROWS, nrow - k * LG_ROWS);
+      for (int q = tid; q < n * (LG_COLS / 4); q += LG_COLS) {
+        const int r = q / (LG_COLS / 4), c = 4 * (q % (LG_COLS / 4));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&sh[b][r][c])),
+                     "l"(h4 + (size_t)((k * LG_ROWS + r) * 32 + l) * MLP_W + c0 + c)
+                     : "memory");
+      }
+      if (tid < n)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&sd[b][tid])),
+                     "l"(dy + (k * LG_ROWS + tid) * 32 + l)
+                     : "memory");
+    }
+    load_commit();
+  };
+  for (int k = 0; k < LG_STAGES - 1; ++k) load(k);
+  float s = 0.f, sb = 0.f;
+  for (int k = 0; k < ns; ++k) {
+    load_wait<LG_STAGES - 2>();
+    __syncthreads();  // stage k has landed and stage k - 1 is read
+    load(k + LG_STAGES - 1);
+    const int b = k % LG_STAGES, n = min(LG_ROWS, nrow - k * LG_ROWS);  // a multiple of 4
+#pragma unroll 4
+    for (int r = 0; r < n; ++r) {
+      const float d = sd[b][r];
+      s += d * sh[b][r][tid];
+      sb += d;
+    }
+  }
+  load_wait<0>();
+  part[(c0 + tid) * 32 + l] = s;
+  if (c0 + tid == 0) part[MLP_W * 32 + l] = sb;
+}
+__global__ void k_mlp_last_sum(const float* part, float* gw5, float* gb5) {
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (w > MLP_W) return;
-  float s = 0.f;
-  for (int b = lane; b < mpad; b += 32) s += dy[b] * (w < MLP_W ? h4[(size_t)b * MLP_W + w] : 1.f);
+  float s = part[w * 32 + lane];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (lane == 0) {
     if (w < MLP_W)
@@ -337,26 +530,65 @@ __global__ void k_mlp_last_grad(const float* dy, const float* h4, int mpad, floa
   }
 }
 
-// dZ4 = dy w5 silu'(Z4): row-major and transposed BF16
-__global__ void k_mlp_dz4(const float* dy, const float* w5, const float* z4, int mpad, __nv_bfloat16* dz,
-                          __nv_bfloat16* dzt) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)mpad * MLP_W) return;
-  const int r = (int)(i / MLP_W), c = (int)(i % MLP_W);
-  const float v = dy[r] * w5[c] * silu_grad_f(z4[i]);
-  dz[i] = __float2bfloat16_rn(v);
-  dzt[(size_t)c * mpad + r] = __float2bfloat16_rn(v);
+// dZ4 = dy w5 silu'(Z4): row-major and transposed BF16, in 64 x 64 tiles
+// through shared memory so that both are written in 128-byte pieces (155 ->
+// 43 us for 65536 rows)
+__global__ void __launch_bounds__(256) k_mlp_dz4(const float* dy, const float* w5, const float* z4, int mpad,
+                                                 __nv_bfloat16* dz, __nv_bfloat16* dzt) {
+  __shared__ float t[64][65];
+  const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;  // mpad % 128 == 0
+  const int c = threadIdx.x & 63;
+  const float w = w5[c0 + c];
+#pragma unroll
+  for (int q = threadIdx.x >> 6; q < 64; q += 4) {
+    const size_t i = (size_t)(r0 + q) * MLP_W + c0 + c;
+    const float v = dy[r0 + q] * w * silu_grad_f(z4[i]);
+    dz[i] = __float2bfloat16_rn(v);
+    t[q][c] = v;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = threadIdx.x >> 5; q < 64; q += 8)
+    *reinterpret_cast<__nv_bfloat162*>(dzt + (size_t)(c0 + q) * mpad + r0 + 2 * lane) =
+        __floats2bfloat162_rn(t[2 * lane][q], t[2 * lane + 1][q]);
 }
 
 // bias gradient: db[j] = sum_b dZ[b][j] from the transposed copy (row j
-// contiguous over the batch); one warp per j
-__global__ void k_mlp_rowsum(const __nv_bfloat16* dzt, int rows, int mpad, float* db) {
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (w >= rows) return;
+// contiguous over the batch) in 32 chains (b mod 32) and a butterfly; a block a
+// row, its segments copied to shared memory ahead of the one warp that sums
+// (114 -> 16 us for 65536 columns, against one warp a row reading them itself)
+constexpr int RS_SEG = 4096;
+__global__ void __launch_bounds__(256) k_mlp_rowsum(const __nv_bfloat16* dzt, int mpad, float* db) {
+  __shared__ __align__(16) __nv_bfloat16 seg[2][RS_SEG];
+  const __nv_bfloat16* row = dzt + (size_t)blockIdx.x * mpad;
+  const int lane = threadIdx.x & 31, ns = (mpad + RS_SEG - 1) / RS_SEG;
+  auto load = [&](int k) {
+    if (k < ns) {
+      const int n = min(RS_SEG, mpad - k * RS_SEG);  // a multiple of 128
+      for (int i = 8 * threadIdx.x; i < n; i += 8 * 256)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&seg[k & 1][i])), "l"(row + k * RS_SEG + i)
+                     : "memory");
+    }
+    load_commit();
+  };
   float s = 0.f;
-  for (int b = lane; b < mpad; b += 32) s += __bfloat162float(dzt[(size_t)w * mpad + b]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) db[w] = s;
+  load(0);
+  for (int k = 0; k < ns; ++k) {
+    load(k + 1);
+    load_wait<1>();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const int n = min(RS_SEG, mpad - k * RS_SEG);
+#pragma unroll 16
+      for (int b = lane; b < n; b += 32) s += __bfloat162float(seg[k & 1][b]);
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x < 32) {
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) db[blockIdx.x] = s;
+  }
 }
 
 // out[i] = sum_s part[s][i] in a fixed order
@@ -369,24 +601,37 @@ __global__ void k_split_reduce(const float* part, int slices, long count, long s
 }
 
 // Adam (Kingma & Ba 2015, bias-corrected) on the FP32 master copy, then the
-// BF16 copies the GEMMs read: w_bf [rows][ld_bf] and optionally its transpose
-// wt_bf [cols][rows]; cols <= ld_bf, the padding columns stay zero
-__global__ void k_mlp_adam(float* w, const float* g, float* m, float* v, long count, int cols, float lr, float b1,
-                           float b2, float eps, float c1, float c2, __nv_bfloat16* w_bf, int ld_bf,
-                           __nv_bfloat16* wt_bf, int rows) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-  w[i] = wi;
-  if (w_bf) {
-    const int r = (int)(i / cols), c = (int)(i % cols);
-    w_bf[(size_t)r * ld_bf + c] = __float2bfloat16_rn(wi);
-    if (wt_bf) wt_bf[(size_t)c * rows + r] = __float2bfloat16_rn(wi);
+// BF16 copies the GEMMs read: wb [rows][ld] and optionally its transpose
+// wt [cols][256]; cols <= ld, the padding columns stay zero. All parameters in
+// one launch: seg lists the weight matrices, the rest (biases, the last layer)
+// has no copies.
+struct AdamSeg {
+  long first, count;
+  int cols, ld;
+  __nv_bfloat16 *wb, *wt;
+};
+struct AdamSegs {
+  AdamSeg s[4];
+};
+__global__ void k_mlp_adam(float* w, const float* g, float* m, float* v, long count, float lr, float b1, float b2,
+                           float eps, float c1, float c2, AdamSegs segs) {
+  const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= count) return;
+  const float gi = g[p];
+  const float mi = b1 * m[p] + (1.f - b1) * gi;
+  const float vi = b2 * v[p] + (1.f - b2) * gi * gi;
+  m[p] = mi;
+  v[p] = vi;
+  const float wi = w[p] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  w[p] = wi;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const AdamSeg& s = segs.s[k];
+    const long i = p - s.first;
+    if (i < 0 || i >= s.count) continue;
+    const int r = (int)(i / s.cols), c = (int)(i % s.cols);
+    s.wb[(size_t)r * s.ld + c] = __float2bfloat16_rn(wi);
+    if (s.wt) s.wt[(size_t)c * MLP_W + r] = __float2bfloat16_rn(wi);
   }
 }
 
@@ -465,17 +710,26 @@ static cudaError_t dmalloc(T** p, size_t count) {
 }
 
 static cudaError_t gemm(tp_mlp* m, GemmArgs a) {
-  static thread_local int attr_dev = -1;
+  static thread_local int attr_dev = -1, sms = 0;
   if (attr_dev != m->device) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+    cudaError_t e = cudaFuncSetAttribute(k_gemm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_gemm_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEMM_SMEM);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
     if (e != cudaSuccess) return e;
     attr_dev = m->device;
   }
   if (a.M % GEMM_BM || a.N % 32 || a.N < 32 || a.N > MLP_W || a.K % GEMM_BK || a.kslices < 1 ||
       (a.K / a.kslices) % GEMM_BK || a.K % a.kslices)
     return cudaErrorInvalidValue;
+  if (a.M > 0 && a.K <= 0) return cudaSuccess;  // nothing to sum
   a.err = m->d_err;
-  k_gemm_tc<<<dim3(a.M / GEMM_BM, a.kslices), GEMM_NT, GEMM_SMEM, m->stream>>>(a);
+  const int tiles = a.M / GEMM_BM;
+  // B in shared memory while it fits; else (and for K slices) the slab ring
+  if (a.kslices == 1 && a.K <= GEMM_KMAX)
+    k_gemm_rows<<<tiles < sms ? tiles : sms, GEMM_NT, GEMM_SMEM, m->stream>>>(a);
+  else
+    k_gemm_ring<<<dim3(tiles, a.kslices), GEMM_NT, GEMM_SMEM, m->stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -561,10 +815,11 @@ static cudaError_t mlp_backward_dev(tp_mlp* m, long n, int rows) {
   cudaError_t e = cudaSuccess;
   const int nb = (rows + 255) / 256;
   k_mlp_loss<<<nb, 256, 0, m->stream>>>(m->y, m->t, n, rows, m->dy, m->lpart);
-  k_sum_fixed<<<1, 32, 0, m->stream>>>(m->lpart, nb, n, m->loss);
-  k_mlp_last_grad<<<(MLP_W + 1 + 7) / 8, 256, 0, m->stream>>>(m->dy, m->H4, rows, m->g + P_W5, m->g + P_B5);
-  k_mlp_dz4<<<(unsigned)(((long)rows * MLP_W + 255) / 256), 256, 0, m->stream>>>(m->dy, m->p + P_W5, m->Z[3], rows,
-                                                                                 m->dZ[0], m->dZT[0]);
+  k_sum_fixed<<<1, 256, 0, m->stream>>>(m->lpart, nb, n, m->loss);
+  // (the chains' sums go through the slice buffer, free until the first GEMM below)
+  k_mlp_last_grad<<<dim3(32, MLP_W / LG_COLS), LG_COLS, 0, m->stream>>>(m->dy, m->H4, rows, m->split);
+  k_mlp_last_sum<<<(MLP_W + 1 + 7) / 8, 256, 0, m->stream>>>(m->split, m->g + P_W5, m->g + P_B5);
+  k_mlp_dz4<<<dim3(rows / 64, MLP_W / 64), 256, 0, m->stream>>>(m->dy, m->p + P_W5, m->Z[3], rows, m->dZ[0], m->dZT[0]);
   e = cudaGetLastError();
   // K slices of the weight-gradient GEMMs: 1024 batch rows each (at most the
   // allocated partial buffers)
@@ -596,7 +851,7 @@ static cudaError_t mlp_backward_dev(tp_mlp* m, long n, int rows) {
       k_split_reduce<<<(unsigned)(((long)MLP_W * in + 255) / 256), 256, 0, m->stream>>>(
           m->split, ks, (long)MLP_W * in, (long)MLP_W * in, m->g + P_W[l]);
     }
-    k_mlp_rowsum<<<MLP_W / 8, 256, 0, m->stream>>>(m->dZT[cur], MLP_W, rows, m->g + P_B[l]);
+    k_mlp_rowsum<<<MLP_W, 256, 0, m->stream>>>(m->dZT[cur], rows, m->g + P_B[l]);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (l == 0 || e != cudaSuccess) break;
     // dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}): B = W_l^T [in][out]
@@ -618,18 +873,19 @@ static cudaError_t mlp_adam_dev(tp_mlp* m, float lr) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   m->adam_t++;
   const float c1 = 1.f - powf(b1, (float)m->adam_t), c2 = 1.f - powf(b2, (float)m->adam_t);
-  for (int l = 0; l < 5; ++l) {
-    const long cw = (long)L_OUT[l] * L_IN[l];
-    __nv_bfloat16* wb = l < 4 ? m->wb[l] : nullptr;
-    __nv_bfloat16* wt = (l >= 1 && l < 4) ? m->wt[l] : nullptr;
-    k_mlp_adam<<<(unsigned)((cw + 255) / 256), 256, 0, m->stream>>>(
-        m->p + P_W[l], m->g + P_W[l], m->m + P_W[l], m->v + P_W[l], cw, L_IN[l], lr, b1, b2, eps, c1, c2, wb,
-        l == 0 ? MLP_IN_PAD : MLP_W, wt, MLP_W);
-    const long cb = L_OUT[l];
-    k_mlp_adam<<<(unsigned)((cb + 255) / 256), 256, 0, m->stream>>>(
-        m->p + P_B[l], m->g + P_B[l], m->m + P_B[l], m->v + P_B[l], cb, 1, lr, b1, b2, eps, c1, c2, nullptr, 0,
-        nullptr, 0);
-  }
+  AdamSegs segs;
+  for (int l = 0; l < 4; ++l)
+    segs.s[l] = {P_W[l], (long)L_OUT[l] * L_IN[l], L_IN[l], l == 0 ? MLP_IN_PAD : MLP_W, m->wb[l], l == 0 ? nullptr : m->wt[l]};
+  k_mlp_adam<<<(unsigned)((P_COUNT + 255) / 256), 256, 0, m->stream>>>(m->p, m->g, m->m, m->v, P_COUNT, lr, b1, b2, eps,
+                                                                      c1, c2, segs);
+  return cudaGetLastError();
+}
+
+static cudaError_t mlp_pack(tp_mlp* m, const float* x, long n, int rows) {
+  cudaError_t e = cudaMemsetAsync(m->XT + (size_t)MLP_IN * rows, 0,
+                                  sizeof(__nv_bfloat16) * (size_t)(MLP_IN_PAD - MLP_IN) * rows, m->stream);
+  if (e != cudaSuccess) return e;
+  k_mlp_pack<<<(rows + 127) / 128, 128, 0, m->stream>>>(x, n, rows, m->X, m->XT);
   return cudaGetLastError();
 }
 
@@ -639,9 +895,7 @@ static cudaError_t mlp_upload_x(tp_mlp* m, const double* x, long n, int rows) {
   cudaError_t e = cudaMemcpyAsync(m->xin, xf.data(), sizeof(float) * xf.size(), cudaMemcpyHostToDevice, m->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);  // xf leaves scope
   if (e == cudaSuccess) {
-    k_mlp_pack<<<(unsigned)(((long)rows * MLP_IN_PAD + 255) / 256), 256, 0, m->stream>>>(m->xin, n, rows, m->X,
-                                                                                           m->XT);
-    e = cudaGetLastError();
+    e = mlp_pack(m, m->xin, n, rows);
   }
   return e;
 }
@@ -809,9 +1063,7 @@ extern "C" int tp_mlp_train_step_device(tp_mlp* m, const float* x_dev, const flo
   cudaError_t e = cudaMemcpyAsync(m->xin, x_dev, sizeof(float) * n * MLP_IN, cudaMemcpyDeviceToDevice, m->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(m->t, t_dev, sizeof(float) * n, cudaMemcpyDeviceToDevice, m->stream);
   if (e == cudaSuccess) {
-    k_mlp_pack<<<(unsigned)(((long)rows * MLP_IN_PAD + 255) / 256), 256, 0, m->stream>>>(m->xin, n, rows, m->X,
-                                                                                           m->XT);
-    e = cudaGetLastError();
+    e = mlp_pack(m, m->xin, n, rows);
   }
   if (e == cudaSuccess) e = mlp_forward_dev(m, rows, true);
   if (e == cudaSuccess) e = mlp_backward_dev(m, n, rows);
