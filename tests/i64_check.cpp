@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "tp_bispec64.cuh"
+#include "tp_pell64.cuh"
 
 using namespace tp;
 typedef long double Q;
@@ -32,6 +33,22 @@ static R plin(const EH& e, R kk, R l2kk) {
   R C = (R)14.4 + (R)325 / (1 + (R)60.5 * q1);
   R r = L / (L + C * qe * qe);
   return (R)e.ehc * e2<R>((R)e.ns * l2kk) * r * r;
+}
+
+struct PRow {
+  double fk, rs, d1, a, b, gam, al, be, xnu, f1, f2, l2fk, l2rs, l2f3c;
+};
+// Takahashi et al. 2012 P(k) with the 2017 correction, as pell_node of tp_cov.cuh
+template <class R>
+static R pnode(const PRow& r, const EH& e, double l2h, double ell, R l2ell) {
+  const R k = (R)ell * (R)r.fk, lk = l2ell + (R)r.l2fk, k3 = k * k * k, pi2 = 9.86960440108935861883449099987615113531L;
+  const R pl = plin<R>(e, k * e2<R>((R)l2h), lk + (R)l2h) * (R)r.d1 * k3 / (2 * pi2);
+  const R ly = lk + (R)r.l2rs, y = k * (R)r.rs, yy = y * y;
+  R ph = (R)r.a * e2<R>(3 * (R)r.f1 * ly) / (1 + (R)r.b * e2<R>((R)r.f2 * ly) + e2<R>((3 - (R)r.gam) * ((R)r.l2f3c + ly)));
+  ph = ph * yy / (yy + (R)r.xnu);
+  const R pq = pl * e2<R>((R)r.be * l2<R>(1 + pl)) / (1 + pl * (R)r.al) * e2<R>(-(y / 4 + yy / 8) * (R)1.442695040888963407359924681L);
+  const R c = e2<R>((R)1.3063 * l2<R>(1 + (R)9.5171e-4 * e2<R>((R)-1.3063 * lk)) - (R)0.62793 * l2<R>(1 + (R)5.1543e-3 * e2<R>((R)-1.1475 * lk)));
+  return c * (2 * pi2 * (pq + ph) / k3);
 }
 
 struct Row {
@@ -171,5 +188,35 @@ int main() {
   const size_t m = va.size();
   printf("nodes %zu\nnode_int_median %g\nnode_dbl_median %g\nnode_int_p99 %g\nnode_dbl_p99 %g\nnode_int_max %g\nnode_dbl_max %g\n", m,
          va[m / 2], vb[m / 2], va[m * 99 / 100], vb[m * 99 / 100], va[m - 1], vb[m - 1]);
+
+  // P(ell) terms over the spectral shapes and scales of a survey's cosmologies
+  va.clear(), vb.clear();
+  const double l2h = log2(.7);
+  for (int it = 0; it < 20000; ++it) {
+    const double ne = -2.6 + U() * 1.4, nc = U() * .6, n2 = ne * ne, om = .15 + .85 * U(), fk = exp2(-13 + U() * 10);
+    PRow r;
+    r.fk = fk, r.rs = exp2(-10 + U() * 14), r.d1 = .04 + .96 * U();
+    r.a = p10(1.5222 + 2.8553 * ne + 2.3706 * n2 + .9903 * ne * n2 + .2250 * n2 * n2 - .6038 * nc + .1749 * (1 - om) * (U() - .5));
+    r.b = p10(-.5642 + .5864 * ne + .5716 * n2 - 1.5474 * nc + .2279 * (1 - om) * (U() - .5));
+    r.gam = .1971 - .0843 * ne + .8460 * nc, r.al = fabs(6.0835 + 1.3373 * ne - .1959 * n2 - 5.5274 * nc);
+    r.be = 2.0379 - .7354 * ne + .3157 * n2 + 1.2490 * ne * n2 + .3980 * n2 * n2 - .1682 * nc, r.xnu = p10(5.2105 + 3.6902 * ne);
+    r.f1 = pow(om, -.0307), r.f2 = pow(om, -.0585);
+    r.l2fk = log2(fk), r.l2rs = log2(r.rs), r.l2f3c = log2(pow(om, .0743) * p10(.3698 + 2.0404 * ne + .8161 * n2 + .5869 * nc));
+    PellNode64 N;
+    pell64_node_make(1., r.fk, r.rs, r.d1, r.a, r.b, r.gam, r.al, r.be, r.xnu, r.f1, r.f2, r.l2fk, r.l2rs, r.l2f3c, l2h, h_i64tab, N);
+    double lo = -60, hi = 60;
+    if (N.ok) pell64_range(r.l2fk, r.l2rs, l2h, lo, hi);
+    // every eighth point an edge of the range
+    const double lg = it % 8 ? fmax(lo, fmin(hi, -1 + U() * 17)) : it % 16 ? lo + .01 : hi - .01, ell = exp2(lg);
+    if (!N.ok) continue;
+    const Q t = pnode<Q>(r, e, l2h, ell, log2l((Q)ell));
+    va.push_back(rel((Q)pell64(N, pell64_point(ell, h_i64tab), tab.data(), h_i64tab) / 1, t));
+    vb.push_back(rel((Q)pnode<double>(r, e, l2h, ell, log2(ell)), t));
+  }
+  std::sort(va.begin(), va.end());
+  std::sort(vb.begin(), vb.end());
+  const size_t k = va.size();
+  printf("pells %zu\npell_int_median %g\npell_dbl_median %g\npell_int_p99 %g\npell_dbl_p99 %g\npell_int_max %g\npell_dbl_max %g\n", k,
+         va[k / 2], vb[k / 2], va[k * 99 / 100], vb[k * 99 / 100], va[k - 1], vb[k - 1]);
   return 0;
 }

@@ -43,3 +43,9 @@ def test_node_is_no_less_accurate_than_the_double_formula(report):
     assert report["nodes"] > 15000
     for q in ("median", "p99", "max"):
         assert report["node_int_" + q] <= report["node_dbl_" + q], q
+
+
+def test_power_spectrum_term_is_no_less_accurate_than_the_double_formula(report):
+    assert report["pells"] > 15000
+    for q in ("median", "p99", "max"):
+        assert report["pell_int_" + q] <= report["pell_dbl_" + q], q

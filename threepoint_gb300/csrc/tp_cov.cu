@@ -33,6 +33,7 @@
 #include "tp_halo.h"
 #include "tp_internal.cuh"
 #include "tp_kernels.cuh"
+#include "tp_pell64.cuh"
 
 namespace tp {
 
@@ -40,26 +41,61 @@ namespace tp {
 // Integrals whose integrand is a weight times a product of P(ell) values
 enum PellKind { K_T1_SQUARE = 0, K_T1_CIRCLE, K_T1_INF, K_T2_A, K_T2_B_SQUARE, K_T2_B_CIRCLE };
 
+// sum of the P(ell) terms of nodes j0 .. j0 + nj - 1 with the FP64 instructions
+static __device__ __noinline__ double pell_nodes_f64(const double* hc, int j0, int nj, double ell, double l2ell,
+                                                     const CosmoK<double>& K) {
+  KSum<double> acc;
+#pragma unroll 2
+  for (int j = j0; j < j0 + nj; ++j) {
+    double v = pell_node<double>(hc, j, ell, l2ell, K);
+    if (v != v) v = 0;
+    acc.add(v);
+  }
+  return acc.s;
+}
 
+// what the FP64 integrands keep in shared memory beside the Halofit rows
+struct PellShared64 {
+  PellNode64 n[NNODE];
+  I64Tables t;
+  double lo, hi;  // ell range of the integer form (empty: none)
+};
+
+// Bound by the integer pipe (98% of the FP64 form's time were its nodes): two
+// entries of the square window 290 -> 28.9 ms, of the infinite T1 176 -> 17.5 ms.
+// FP64: the integer form (tp_pell64.cuh) with the FP64 instructions as the
+// reference form of the cubature's ties and outside the integer form's domain
 template <typename R, int DIM, int KIND>
 struct PellProd {
   static constexpr int NCH = 8;  // node chunks of 12 per P(ell)
   static constexpr int NL = (KIND <= K_T1_INF) ? 3 : 1;
   static constexpr int G = NL * NCH;
   static constexpr int PD = 1;
-  static constexpr int MINB = 1;
-  static constexpr bool CLUSTER16 = false;
+  static constexpr int MINB = sizeof(R) == 8 && DIM < 6 ? 2 : 1;
+  // few costly integrals (the oscillating 2-D term: two entries 40.9 -> 28.9 ms
+  // in 16-CTA clusters instead of 8); FP32 points are cheap beside the sweeps
+  static constexpr bool CLUSTER16 = sizeof(R) == 8 && (DIM == 2 || DIM == 3);
   static constexpr int NS = NL;
   __device__ static int slot(int g) { return g / NCH; }
   static constexpr int CH = (DIM == 6) ? 2 : 8;
-  struct Rec {
+  struct RecF {
     R ell[3], l2ell[3];
     double wt;
     int valid, los;
   };
+  struct RecD {
+    double ell[NL], l2ell[NL];  // l2ell: FP64 form
+    double wt;
+    int valid, los, f64form, pad;
+    Pell64 p[NL];
+  };
+  typedef typename std::conditional<sizeof(R) == 4, RecF, RecD>::type Rec;
   static constexpr int REC = (int)sizeof(Rec);
   const int* job_order = nullptr;
-  static constexpr size_t PSMEM = sizeof(R) * HC_COUNT * NNODE + sizeof(CosmoK<R>) + 64;
+  static constexpr bool REF = sizeof(R) == 8;
+  int ref;
+  static constexpr size_t HC_BYTES = sizeof(R) * HC_COUNT * NNODE;
+  static constexpr size_t PSMEM = HC_BYTES + (REF ? sizeof(PellShared64) : 0) + sizeof(CosmoK<R>) + 64;
 
   const CovJob* jobs;
   const R* hcoef;  // this cosmology's Halofit node table
@@ -75,12 +111,36 @@ struct PellProd {
   double th[6], lmin, lmax;
   int loaded;
 
+  __device__ PellShared64& shared64() const { return *(PellShared64*)((char*)s_hc + HC_BYTES); }
+  __device__ void load64() {
+    PellShared64& s = shared64();
+    for (int i = threadIdx.x; i < (int)(sizeof(I64Tables) / 4); i += blockDim.x)
+      ((uint32_t*)&s.t)[i] = ((const uint32_t*)&d_i64tab)[i];
+    const auto row = [&](int q, int j) { return (double)s_hc[q * NNODE + j]; };
+    for (int j = threadIdx.x; j < NNODE; j += blockDim.x)
+      pell64_node_make(row(HC_W, j), row(HC_INVFK, j), row(HC_RS, j), row(HC_D1SQ, j), row(HC_A, j), row(HC_B, j),
+                       row(HC_GAM, j), row(HC_ALPHA, j), row(HC_BETA, j), row(HC_XNU, j), row(HC_F1, j), row(HC_F2, j),
+                       row(HC_L2INVFK, j), row(HC_L2RS, j), row(HC_L2F3C, j), ck.l2h, d_i64tab, s.n[j]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double lo = -60, hi = 60;
+      for (int j = 0; j < NNODE; ++j)
+        if (s.n[j].ok) pell64_range(row(HC_L2INVFK, j), row(HC_L2RS, j), ck.l2h, lo, hi);
+      s.lo = exp2(lo + 0.01);
+      s.hi = lo < hi ? exp2(hi - 0.01) : 0.0;
+    }
+  }
+
   __device__ void begin_job(int job, char* psmem, double* xmin, double* xmax) {
     s_hc = (R*)psmem;
     if (!loaded) {
       __syncthreads();
       for (int i = threadIdx.x; i < HC_COUNT * NNODE; i += blockDim.x) s_hc[i] = hcoef[i];
       __syncthreads();
+      if constexpr (REF) {
+        load64();
+        __syncthreads();
+      }
       loaded = 1;
     }
     const CovJob& J = jobs[job];
@@ -156,9 +216,23 @@ struct PellProd {
     r.valid = !zero && wt != 0.0;
     r.los = r.valid && !constant_ps;
     r.wt = wt;
-    for (int i = 0; i < NL; ++i) {
-      r.ell[i] = (R)ell[i];
-      r.l2ell[i] = r.valid ? (R)log2(ell[i]) : (R)0;
+    if constexpr (sizeof(R) == 4) {
+      for (int i = 0; i < NL; ++i) {
+        r.ell[i] = (R)ell[i];
+        r.l2ell[i] = r.valid ? (R)log2(ell[i]) : (R)0;
+      }
+    } else if (r.los) {
+      const PellShared64& s = shared64();
+      bool in = ck.c64.ok && !ref;
+      for (int i = 0; i < NL; ++i) in = in && ell[i] >= s.lo && ell[i] <= s.hi;
+      r.f64form = !in;
+      for (int i = 0; i < NL; ++i) {
+        r.ell[i] = ell[i];
+        if (in)
+          r.p[i] = pell64_point(ell[i], s.t);
+        else
+          r.l2ell[i] = log2(ell[i]);
+      }
     }
     return r.los;
   }
@@ -166,15 +240,28 @@ struct PellProd {
   __device__ void group(const char* recp, int g, double* pv) {
     const Rec& r = *(const Rec*)recp;
     const int i = g / NCH, ch = g % NCH;
-    KSum<R> acc;
     const int j0 = ch * (NNODE / NCH);
+    if constexpr (sizeof(R) == 4) {
+      KSum<R> acc;
 #pragma unroll 2
-    for (int j = j0; j < j0 + NNODE / NCH; ++j) {
-      R v = pell_node<R>(s_hc, j, r.ell[i], r.l2ell[i], ck);
-      if (v != v) v = (R)0;
-      acc.add(v);
+      for (int j = j0; j < j0 + NNODE / NCH; ++j) {
+        R v = pell_node<R>(s_hc, j, r.ell[i], r.l2ell[i], ck);
+        if (v != v) v = (R)0;
+        acc.add(v);
+      }
+      pv[0] = (double)acc.s;
+    } else if (r.f64form) {
+      pv[0] = pell_nodes_f64(s_hc, j0, NNODE / NCH, r.ell[i], r.l2ell[i], ck);
+    } else {
+      const PellShared64& s64 = shared64();
+      double s = 0;
+      for (int j = j0; j < j0 + NNODE / NCH; ++j) {
+        double v = s64.n[j].ok ? pell64(s64.n[j], r.p[i], ck.c64.p, s64.t)
+                               : pell_nodes_f64(s_hc, j, 1, r.ell[i], log2(r.ell[i]), ck);
+        if (v == v) s += v;
+      }
+      pv[0] = s;
     }
-    pv[0] = (double)acc.s;
   }
 
   __device__ void finalize(const char* recp, const double* sum, double* fv) {
@@ -569,7 +656,7 @@ static int run_pell_kind(tp_ctx* ctx, int cosmo, const JobSet& js, double theta_
   pol.thetaMax = theta_max;
   pol.thetaMaxY = theta_max_y;
   pol.norm = norm;
-  return run_jobs<DIM>(ctx, pol, js.jobs, rel_tol, 0, res, bad);
+  return run_jobs<DIM>(ctx, pol, js.jobs, rel_tol, PellProd<R, DIM, KIND>::CLUSTER16 ? 16 : 0, res, bad);
 }
 
 template <typename R>
