@@ -368,20 +368,21 @@ TP_TABLE_KERNEL k_eh_table(const CosmoDev* cos, const EHConst* eh, double* ehg, 
 }
 
 // r_sigma by bisection on D1 sigma(1/k) = 1, then n_eff and ncur
-// (bispectrum.cu:202-212, 870-903). One warp takes RS_BINS adjacent redshift
-// bins of a cosmology; lane b < RS_BINS holds bin b's bisection as a state
+// (bispectrum.cu:202-212, 870-903). One warp takes `bins` (a power of two, at
+// most RS_BINS) adjacent redshift bins of a cosmology; lane b < bins holds bin b's bisection as a state
 // machine that advances one iteration of the one-bin loops per round. sigma(R)
 // does not depend on the bin, and while adjacent bins' brackets coincide they
 // ask for sigma at bitwise the same k: each round the warp evaluates every
 // distinct k once (all 32 lanes in the trapezoid sums) and hands the value to
 // the bins that asked for it. Every bin sees the same sequence of values and
-// makes the same decisions as alone, with ~40% fewer sigma(R) integrals.
+// makes the same decisions as alone, with ~40% fewer sigma(R) integrals at RS_BINS.
 constexpr int RS_BINS = 8;
 static_assert(NZ % RS_BINS == 0 && RS_BINS <= 32, "bins per warp");
 
-TP_TABLE_KERNEL k_rsigma(const CosmoDev* cos, const EHConst* eh, TablesDev* tab, const double* ehg_all, int n) {
+TP_TABLE_KERNEL k_rsigma(const CosmoDev* cos, const EHConst* eh, TablesDev* tab, const double* ehg_all, int n,
+                         int bins) {
   const unsigned FULL = 0xffffffffu;
-  const int ci = blockIdx.x / (NZ / RS_BINS), b0 = (blockIdx.x % (NZ / RS_BINS)) * RS_BINS;
+  const int ci = blockIdx.x / (NZ / bins), b0 = (blockIdx.x % (NZ / bins)) * bins;
   if (ci >= n) return;
   const int lane = threadIdx.x & 31;
   const CosmoDev c = tables_cosmo(cos[ci]);
@@ -389,7 +390,7 @@ TP_TABLE_KERNEL k_rsigma(const CosmoDev* cos, const EHConst* eh, TablesDev* tab,
   TablesDev& t = tab[ci];
   const double* pk = t.pk;
   const double* ehg = ehg_all + (size_t)ci * EHG_N;
-  const bool mine = lane < RS_BINS;
+  const bool mine = lane < bins;
   const int bin = b0 + (mine ? lane : 0);
   const double D1 = t.D1[bin];
   // phase 0: k1 halving (<= 100 steps), 1: k2 doubling (<= 100), 2: bisection
@@ -451,7 +452,7 @@ TP_TABLE_KERNEL k_rsigma(const CosmoDev* cos, const EHConst* eh, TablesDev* tab,
   const double rs = (c.sigma8 >= 1e-8) ? (bad ? NAN : 1. / k) : 0.0;
   // n_eff and ncur need sigma at each bin's own radius: one bin after another
   double s2 = NAN, s3 = NAN;
-  for (int b = 0; b < RS_BINS; ++b) {
+  for (int b = 0; b < bins; ++b) {
     const double rb = __shfl_sync(FULL, rs, b);
     if (!isfinite(rb)) continue;
     const double v2 = warp_sigmam(c, e, pk, rb, 2, ehg);
@@ -463,6 +464,152 @@ TP_TABLE_KERNEL k_rsigma(const CosmoDev* cos, const EHConst* eh, TablesDev* tab,
     t.r_sigma[bin] = rs;
     t.n_eff[bin] = -3. + 2. * (D1 * s2) * (D1 * s2);
     t.ncur[bin] = d1 * d1 + 4. * s3 * D1 * D1;
+  }
+}
+// ---- the wide forms: few cosmologies -----------------------------------------
+// One cosmology's serial chains (RK4 steps, bisections) in 8-32 blocks of a warp
+// leave the SMs idle and set the time of a sampler's step. Up to TABLES_WIDE
+// cosmologies the growth integral therefore takes a warp per redshift bin, the
+// normalisation a block, and k_rsigma fewer bins a warp; sums and chains are
+// those of the forms above operation by operation, and so are the results.
+// Measured (GB300): set_cosmologies of 1 cosmology 22.7 -> 5.9 ms (k_rsigma 16.5
+// -> 3.0, growth 4.3 -> 1.15, norm 2.5 -> 0.76), 4: 27.4 -> 8.7, 16: 29.2 -> 21.8,
+// 24: 33.4 -> 31.8 ms; at 32 the narrow forms do less work (37.1 against 38.0).
+constexpr int TABLES_WIDE = 24;
+// k_rsigma's bins a warp there: as few as leave about ten warps an SM (one
+// cosmology 5.9 / 8.4 / 12.1 ms with 1 / 2 / 4 bins, twelve 21.0 / 18.0 / 18.8,
+// twenty-four 39.3 / 33.7 / 31.8)
+constexpr int RS_WIDE_WARPS = 1536;
+
+// d_lgr by a warp: the lanes evaluate the coefficients of 32 steps' right-hand
+// sides (exp and pow do not depend on y), then all take the steps, with
+// d_lgr's roundings written out
+__device__ double warp_lgr(const CosmoDev& c, double z) {
+  __shared__ double sc[32][9];
+  const int lane = threadIdx.x & 31;
+  double a = 1. / (1. + z), a0 = 1. / 1100.;
+  double yp = -1., y0 = 1, y1 = 0;
+  int n = 10;
+  auto coef = [&](double la, double* o) {
+    double ea = exp(la);
+    double ap = pow(ea, -3. * c.w);
+    o[0] = __dmul_rn(-0.5, __fma_rn(5.0, c.om, __dmul_rn(__dmul_rn(__dsub_rn(5.0, __dmul_rn(3.0, c.w)), c.ow), ap)));
+    o[1] = __dmul_rn(__dmul_rn(__dmul_rn(1.5, __dsub_rn(1.0, c.w)), c.ow), ap);
+    o[2] = __fma_rn(c.ow, ap, c.om);
+  };
+  for (int it = 0; it < 20; ++it) {
+    n *= 2;
+    double h = (log(a) - log(a0)) / n;
+    double x = log(a0);
+    y0 = 1.;
+    y1 = 0.;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      double xl = x;
+      for (int s = 0; s < lane; ++s) xl += h;
+      __syncwarp();
+      coef(xl, sc[lane]);
+      coef(xl + 0.5 * h, sc[lane] + 3);
+      coef(xl + h, sc[lane] + 6);
+      x = __shfl_sync(0xffffffffu, xl + h, 31);
+      __syncwarp();
+      const int m = min(32, n - i0);
+      for (int s = 0; s < m; ++s) {
+        const double* q = sc[s];
+        auto rhs = [&](const double* o, double u0, double u1) {
+          return __ddiv_rn(__fma_rn(o[0], u1, -__dmul_rn(o[1], u0)), o[2]);
+        };
+        const double k10 = __dmul_rn(h, y1), r1 = rhs(q, y0, y1), k11 = __dmul_rn(h, r1);
+        const double a0_ = __dadd_rn(y0, 0.5 * k10), a1_ = __dadd_rn(y1, 0.5 * k11);
+        const double k21 = __dmul_rn(h, rhs(q + 3, a0_, a1_));
+        const double b0_ = __dadd_rn(y0, 0.5 * __dmul_rn(h, a1_)), b1_ = __dadd_rn(y1, 0.5 * k21);
+        const double k30 = __dmul_rn(h, b1_), k31 = __dmul_rn(h, rhs(q + 3, b0_, b1_));
+        const double c0_ = __dadd_rn(y0, k30), c1_ = __dadd_rn(y1, k31);
+        const double r4 = rhs(q + 6, c0_, c1_);
+        y0 = __dadd_rn(y0, __dadd_rn(__ddiv_rn(__fma_rn(h, y1, __dmul_rn(h, c1_)), 6.), __ddiv_rn(__fma_rn(h, a1_, k30), 3.)));
+        y1 = __dadd_rn(y1, __dadd_rn(__ddiv_rn(__fma_rn(h, r4, k11), 6.), __ddiv_rn(__dadd_rn(k21, k31), 3.)));
+      }
+    }
+    if (!isfinite(y0) || fabs(y0 / yp - 1.) < 0.1 * EPS) break;
+    yp = y0;
+  }
+  return a * y0;
+}
+// lgr at the bin centres and (the last block of a cosmology) at z = 0
+__global__ void __launch_bounds__(32) k_growth_wide(const CosmoDev* cos, TablesDev* tab, int n) {
+  const int ci = blockIdx.x / (NZ + 1), i = blockIdx.x % (NZ + 1);
+  if (ci >= n) return;
+  const CosmoDev c = cos[ci];
+  const double v = warp_lgr(c, i == NZ ? 0. : (i + 0.5) * (c.zmax / NZ));
+  if (threadIdx.x == 0) {
+    if (i == NZ)
+      tab[ci].lgr0 = v;
+    else
+      tab[ci].D1[i] = v;
+  }
+}
+__global__ void k_growth_scale(TablesDev* tab) { tab[blockIdx.x].D1[threadIdx.x] /= tab[blockIdx.x].lgr0; }
+
+// k_norm by a block: warp w evaluates every sixteenth of the points a lane of
+// warp_sigmam sums one after the other, and every warp adds them in that order
+// (the integrand's last factor W in the sum's FMA, as there)
+constexpr int NORM_WARPS = 16;
+__global__ void __launch_bounds__(32 * NORM_WARPS) k_norm_wide(const CosmoDev* cos, EHConst* eh, TablesDev* tab, int n) {
+  __shared__ double sv[NORM_WARPS][32], sw[NORM_WARPS][32];
+  const int ci = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (ci >= n) return;
+  const CosmoDev c = tables_cosmo(cos[ci]);
+  const EHConst e = eh[ci];
+  double sigma = 0;
+  if (!(c.sigma8 < 1e-8)) {
+    const double r = 8.;
+    auto f = [&](double k, double& w) {
+      w = d_window(k * r, 0);
+      return k * k * k * d_linear_pk(c, e, tab[ci].pk, k) * w;
+    };
+    double k1 = 2. * PI / r, k2 = 2. * PI / r;
+    double xx = 0, xxpp = -1.0;
+    for (int outer = 0; outer < 40; ++outer) {
+      k1 = k1 / 10.0;
+      k2 = k2 * 2.0;
+      double a = log(k1), b = log(k2);
+      double xxp = -1.0;
+      int m = 2;
+      double w1, w2;
+      const double x1 = f(k1, w1), x2 = f(k2, w2);
+      double ends = 0.5 * __fma_rn(x1, w1, __dmul_rn(x2, w2));
+      double sum = 0;
+      for (int inner = 0; inner < 21; ++inner) {
+        m = m * 2;
+        double hh = (b - a) / (double)m;
+        double part = 0;
+        // first level: all three interior points; then the odd ones
+        const int cnt = m == 4 ? 3 : m / 2;
+        for (int q0 = 0; q0 < cnt; q0 += 32 * NORM_WARPS) {
+          const int q = q0 + 32 * warp + lane;
+          __syncthreads();
+          if (q < cnt) {
+            double t = __fma_rn(hh, (double)(m == 4 ? 1 + q : 2 * q + 1), a);
+            sv[warp][lane] = f(exp(t), sw[warp][lane]);
+          }
+          __syncthreads();
+          for (int w = 0; w < NORM_WARPS && q0 + 32 * w + lane < cnt; ++w) part = __fma_rn(sv[w][lane], sw[w][lane], part);
+        }
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        sum += part;
+        xx = (sum + ends) * hh;
+        if (!isfinite(xx) || fabs((xx - xxp) / xx) < EPS) break;
+        xxp = xx;
+      }
+      if (!isfinite(xx) || fabs((xx - xxpp) / xx) < EPS) break;
+      xxpp = xx;
+    }
+    sigma = sqrt(xx / (2.0 * PI * PI));
+  }
+  if (threadIdx.x == 0) {
+    double norm = c.sigma8 / sigma;
+    tab[ci].norm = norm;
+    tab[ci].dz = c.zmax / NZ;
+    eh[ci].ehc = e.ehc * norm * norm;
   }
 }
 
@@ -835,11 +982,20 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
     carveout_set = dev;
   }
   k_eh_table<<<(unsigned)((long)n * EHG_N / 32), 32, 0, s>>>(d_cos, d_eh, d_ehg, n);
-  k_norm<<<n, 32, 0, s>>>(d_cos, d_eh, d_tab, n);
+  const bool wide = n <= TABLES_WIDE;
+  int bins = wide ? 1 : RS_BINS;
+  while (bins < RS_BINS && n * (NZ / bins) > RS_WIDE_WARPS) bins *= 2;
+  if (wide) {
+    k_growth_wide<<<n * (NZ + 1), 32, 0, s>>>(d_cos, d_tab, n);
+    k_growth_scale<<<n, NZ, 0, s>>>(d_tab);
+    k_norm_wide<<<n, 32 * NORM_WARPS, 0, s>>>(d_cos, d_eh, d_tab, n);
+  } else {
+    k_norm<<<n, 32, 0, s>>>(d_cos, d_eh, d_tab, n);
+  }
   k_fk<<<n * (NZ / 32), 32, 0, s>>>(d_cos, d_tab, n);
   k_g<<<n * (NZ / 32), 32, 0, s>>>(d_cos, d_nz, nz_stride, d_tab, n);
-  k_growth<<<n * (NZ / 32), 32, 0, s>>>(d_cos, d_tab, n);
-  k_rsigma<<<(unsigned)((long)n * (NZ / RS_BINS)), 32, rsigma_smem, s>>>(d_cos, d_eh, d_tab, d_ehg, n);
+  if (!wide) k_growth<<<n * (NZ / 32), 32, 0, s>>>(d_cos, d_tab, n);
+  k_rsigma<<<(unsigned)((long)n * (NZ / bins)), 32, wide ? 0 : rsigma_smem, s>>>(d_cos, d_eh, d_tab, d_ehg, n, bins);
   k_node_coefs<<<n * (NNODE / 32), 32, 0, s>>>(d_cos, d_tab, d_ncoef, d_ncoef_f, d_fcoef_f, d_hcoef, d_hcoef_f, n);
   k_finish<<<n, 32, 0, s>>>(d_cos, d_eh, d_tab, d_ncoef, d_ncoef_f, d_fcoef_f, d_wscale64, d_wscale32, d_ck64, d_ck32,
                             n);
