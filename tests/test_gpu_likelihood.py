@@ -115,3 +115,23 @@ class _Indexable:
 
     def get_string(self, s, k):
         return self.b.get_string(s, k)
+
+
+# one row, rows beside the block's 256 and its multiples; batches on both sides
+# of the staging size (256 KiB). spd()'s condition number is below 20: the sums of
+# n products and the factorisation lose at most n 20 2^-53 times a few
+@pytest.mark.parametrize("n,b", [(1, 1), (31, 4096), (33, 990), (255, 3), (257, 127), (257, 128), (700, 60)])
+def test_chi2_at_block_and_staging_edges(n, b):
+    import threepoint_gb300 as tp
+
+    rng = np.random.default_rng(n + b)
+    cov, data = spd(n, n), rng.normal(size=n) * 1e-10
+    models = data + rng.normal(size=(b, n)) * 1e-10
+    lk = tp.Likelihood(data, cov)
+    try:
+        z = np.linalg.solve(np.linalg.cholesky(cov), (models - data).T)
+        ref = (z * z).sum(0)
+        for _ in range(2):
+            assert np.abs(lk.chi2(models) / ref - 1).max() <= 100 * n * 2.0 ** -53 + 1e-14
+    finally:
+        lk.close()
