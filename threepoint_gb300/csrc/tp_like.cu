@@ -100,7 +100,7 @@ __global__ void k_transpose(const double* x, double* xt, int n) {
 // z = X (m - d), chi2 = sum z_i^2, summed in a fixed order. A thread a row of
 // X, read from the transpose so that a warp's loads are coalesced and sixteen
 // are in flight; large batches are bound by the FP64 pipe (n^2 / 2 DFMA a
-// model: 4096 models of 700 in 1.97 ms, 1.93 its floor), small ones by a row's chain
+// model: 4096 models of 700 in 1.97 ms, the pipe's rate), small ones by a row's chain
 __global__ void __launch_bounds__(CNT) k_chi2(const double* xt, const double* data, const double* models, long ld,
                                               int n, double* chi2) {
   extern __shared__ double sm[];
