@@ -811,7 +811,7 @@ __device__ inline bool zrow64(const TablesDev& t, const CosmoDev& c, const Cosmo
   const double ne = t.n_eff[i0] * w0 + t.n_eff[i1] * w1;
   const double s = rs / fK, hf = c.h / fK, zp = 1.0 + z, ds = D1 * c.sigma8;
   if (!(K.c64.ok && K.n64[0].ok && z <= 10. && s > 0x1p-27 && s < 0x1p36 && hf > 0x1p-60 && hf < 0x1p60 && ds > 1e-4 &&
-        ds < 1e4 && ne > -5 && ne < 1 && D1 > 1e-30 && D1 < 1e30))
+        ds < 1e4 && ne > -5 && ne < 1 && D1 > 1e-18 && D1 < 1e18 && fabs(c.w) < 50))
     return true;
   auto L = [&](double v) { return i64_log2(v, d_i64tab); };        // Q57
   auto X = [&](double v) { return i64_fix<52>(v); };               // Q52
@@ -838,8 +838,11 @@ __device__ inline bool zrow64(const TablesDev& t, const CosmoDev& c, const Cosmo
   N.l2bn = X(L10 * (-3.428 + ls * (-2.681 + ls * (1.624 + ls * -0.095))));
   N.mun = Q(L10 * (15.312 + ne * (22.977 + ne * (10.9579 + ne * 1.6586))), 59);
   N.nun = Q(L10 * (1.347 + ne * (1.246 + ne * 0.4525)), 59);
-  N.kmn = (int64_t)((uint64_t)X(L10 * (-2.605 + ls * (-2.434 + ls * 5.71))) - (N.mun >> 1));
-  N.knn = (int64_t)((uint64_t)X(L10 * (-4.468 + ls * (-3.08 + ls * 1.035))) - (N.nun >> 1));
+  const double l2mn = L10 * (-2.605 + ls * (-2.434 + ls * 5.71)), l2nn = L10 * (-4.468 + ls * (-3.08 + ls * 1.035));
+  N.kmn = (int64_t)((uint64_t)X(l2mn) - (N.mun >> 1));
+  N.knn = (int64_t)((uint64_t)X(l2nn) - (N.nun >> 1));
+  // the exponents' range (pow_ok)
+  ok = ok && fabs(l2mn) + 63 * ((double)N.mun * 0x1p-59) < 2040 && fabs(l2nn) + 63 * ((double)N.nun * 0x1p-59) < 2040;
   Sf v = E(X(L10 * (0.159 - 1.107 * ne)) + s52);
   N.cns = v.m, N.ecns = v.e;
   v = sf_norm(sf_mul(sf_norm(sf_mul(v, v)), v));

@@ -73,11 +73,18 @@ struct Tri64 {
   double f2t[3];
 };
 
-// log2 of a positive normal double, Q57, within 2^-57
+// log2 of a positive normal double in [2^-64, 2^64), Q57, within 2^-57
 TP_HD int64_t i64_log2(double x, const I64Tables& t) {
   const Sf a = sf_from(x);
   return (int64_t)(((uint64_t)(a.e + 63) << 57) + (uint64_t)((i64_log2m(a.m, t.rc, t.lc) + 16) >> 5));
 }
+// of any positive normal double, in units of 2^-(57 - SH)
+template <int SH>
+TP_HD int64_t i64_log2_sh(double x, const I64Tables& t) {
+  const Sf a = sf_from(x);
+  return (int64_t)((uint64_t)(int64_t)(a.e + 63) << (57 - SH)) + ((i64_log2m(a.m, t.rc, t.lc) + 16) >> (5 + SH));
+}
+TP_HD int64_t i64_log2_q52(double x, const I64Tables& t) { return i64_log2_sh<5>(x, t); }
 
 // triangle (ell1, ell2, ell3); f2t = F2_tree(1,2,3), (2,3,1), (3,1,2). Returns
 // ok: every ell inside [lo, hi] (and so inside the fixed-point range)
@@ -114,8 +121,10 @@ TP_HD bool tri64_make(double l1, double l2, double l3, const double* f2t, double
   return true;
 }
 
-TP_HD bool q59_ok(double c) { return c >= 0 && c < 31.9; }
 TP_HD bool sf_ok(double c) { return c > 1e-280 && c < 1e280; }
+TP_HD bool q59_ok(double c) { return c >= 0 && c < 15.9; }
+// a c q^m whose base-2 exponent stays inside Q52 over the node's whole range of log2 q (-63 to 63)
+TP_HD bool pow_ok(double c, double m) { return sf_ok(c) && m >= 0 && fabs(log2(c)) + 63 * m < 2040; }
 
 // node row from the FP64 coefficients (NC_* values)
 TP_HD void node64_make(double w, double s, double hf, double ana, double anr, double anc, double bn, double cn,
@@ -127,23 +136,23 @@ TP_HD void node64_make(double w, double s, double hf, double ana, double anr, do
   N.ens = en * s;
   const double pns = pn * s, cns = cn * s, f = d1sq * fn * s * s, h = hn * s * s, g = gn * s;
   N.ok = !tree && s > 0x1p-27 && s < 0x1p36 && hf > 0x1p-60 && hf < 0x1p60 && sf_ok(anr) && anr < 16 && q59_ok(anc) &&
-         q59_ok(ald) && betab >= 0 && betab < 15.5 && q59_ok(mun) && q59_ok(nun) && sf_ok(bn) && sf_ok(mn) &&
-         sf_ok(nn) && fabs(ana) < 900 && fabs(ala) < 900 && sf_ok(cns) && cns > 1e-80 && cns < 1e80 && sf_ok(f) && sf_ok(d1sq) &&
+         q59_ok(ald) && betab >= 0 && betab < 15.5 && mun < 31.9 && nun < 31.9 && pow_ok(bn, betab * 1.017) && pow_ok(mn, mun) &&
+         pow_ok(nn, nun) && fabs(ana) < 900 && fabs(ala) < 900 && sf_ok(cns) && cns > 1e-80 && cns < 1e80 && sf_ok(f) && sf_ok(d1sq) &&
          sf_ok(h) && sf_ok(g) && pns > 1e-80 && pns < 1e80;
   if (!N.ok) return;
   N.l2s = i64_log2(s, t);
   N.l2hf = i64_log2(hf, t);
   N.anc = (uint64_t)i64_fix<59>(anc);
   N.ald = (uint64_t)i64_fix<59>(ald);
-  N.l2anr = i64_log2(anr, t) >> 5;
+  N.l2anr = i64_log2_q52(anr, t);
   N.ana = i64_fix<52>(ana);
   N.ala = i64_fix<52>(ala);
   N.betab = (uint64_t)i64_fix<60>(betab * 0.5) << 1;
-  N.l2bn = i64_log2(bn, t) >> 5;
+  N.l2bn = i64_log2_q52(bn, t);
   N.mun = (uint64_t)i64_fix<58>(mun) << 1;
   N.nun = (uint64_t)i64_fix<58>(nun) << 1;
-  N.kmn = (int64_t)((uint64_t)(i64_log2(mn, t) >> 5) - (N.mun >> 1));
-  N.knn = (int64_t)((uint64_t)(i64_log2(nn, t) >> 5) - (N.nun >> 1));
+  N.kmn = (int64_t)((uint64_t)i64_log2_q52(mn, t) - (N.mun >> 1));
+  N.knn = (int64_t)((uint64_t)i64_log2_q52(nn, t) - (N.nun >> 1));
   Sf v = sf_from(cns);
   N.cns = v.m, N.ecns = v.e;
   v = sf_norm(sf_mul(sf_norm(sf_mul(v, v)), v));
@@ -173,7 +182,9 @@ TP_HD bool p64_cell(int i, double omh2, double sa, double one_m_sa, double sh043
   double x[6], d[6];
   int64_t y0 = 0;
   const int64_t l0 = (int64_t)((uint64_t)P64_LO << 57) + ((int64_t)i << 50);
-  const int64_t lehc = i64_log2(ehc, t), nsq = i64_fix<56>(ns);
+  // log2 P within +-512 (Q51 of eight times it)
+  if (!(fabs(log2(ehc)) < 80)) return false;
+  const int64_t lehc = i64_log2_sh<3>(ehc, t), nsq = i64_fix<56>(ns);
   for (int k = 0; k < 6; ++k) {
     const int64_t lk = l0 + ((int64_t)tk[k] << 34);  // log2(k h), Q57
     const double kk = sf_to(i64_exp2(lk >> 5, t.ex2));
@@ -183,11 +194,12 @@ TP_HD bool p64_cell(int i, double omh2, double sa, double one_m_sa, double sh043
     const double L = log(2.718281828 + c184 * q);
     const double C = 14.4 + 325.0 / (1.0 + 60.5 * exp2(1.11 * log2(q)));
     const double r = L / (L + C * q * q);
+    if (!(r > 0x1p-100)) return false;
     // n_s log2 k in Q54 from Q57 and Q56
     const uint64_t al = (uint64_t)(lk < 0 ? -lk : lk), an = (uint64_t)(nsq < 0 ? -nsq : nsq);
     int64_t pw = (int64_t)(i64_mulhi_exact(al, an) << 5) + (int64_t)((al * an) >> 59);
     if ((lk < 0) != (nsq < 0)) pw = -pw;
-    const int64_t y = (lk >> 1) - (lehc >> 3) - pw - (i64_log2(r, t) >> 2);  // Q51
+    const int64_t y = (lk >> 1) - lehc - pw - i64_log2_sh<2>(r, t);  // Q51
     if (k == 0) y0 = y;
     x[k] = tk[k] * 0x1p-16;
     d[k] = (double)(y - y0) * 0x1p-54;

@@ -59,8 +59,8 @@ TP_HD void pell64_node_make(double w, double invfk, double rs, double d1sq, doub
   N.s2 = q59_even(f2), N.n2 = f2 < 0 ? -1 : 0;
   N.s3 = q59_even(s3), N.n3 = s3 < 0 ? -1 : 0;
   N.be = q59_even(beta), N.nb = beta < 0 ? -1 : 0;
-  N.k1 = pell64_off(0.0, s1, 0.0, N.s1) + (i64_log2(a, t) >> 5);
-  N.k2 = pell64_off(0.0, f2, 0.0, N.s2) + (i64_log2(b, t) >> 5);
+  N.k1 = pell64_off(0.0, s1, 0.0, N.s1) + i64_log2_q52(a, t);
+  N.k2 = pell64_off(0.0, f2, 0.0, N.s2) + i64_log2_q52(b, t);
   N.k3 = pell64_off(0.0, s3, l2f3c, N.s3);
   Sf v = sf_from(cpl);
   N.cpl = v.m, N.ecpl = v.e;
