@@ -102,7 +102,7 @@ __device__ __forceinline__ R plin(const CosmoK<R>& K, R kk, R l2kk) {
     R didx = (lnk - K.ln_kmin) * K.inv_dk;
     if (didx <= (R)0) return (R)K.pk[0];
     if (didx >= (R)(NK - 1)) return (R)K.pk[NK - 1];
-    int idx = (int)didx;
+    int idx = sizeof(R) == 8 && !(didx > (R)0) ? 0 : (int)didx;  // an FP64 NaN converts to INT_MIN, an FP32 one to 0
     R f = didx - (R)idx;
     return (R)K.pk[idx] * ((R)1 - f) + (R)K.pk[idx + 1] * f;
   }
@@ -718,7 +718,7 @@ __device__ __forceinline__ TriF trif_scaled(const TriF& T, float sc, float l2sc)
 // Mid-bin two-point interpolation of a z table at fractional bin position fb
 // (cuda_version/bispectrum.cu:335-437) with the lower neighbour clamped at bin 0.
 __host__ __device__ inline void interp_mid_w(double fb, int& i0, int& i1, double& w0, double& w1) {
-  int idx = (int)fb;
+  int idx = fb > 0 ? (int)fb : 0;  // (NaN converts to INT_MIN)
   double didx = fb - idx;
   if (idx > NZ - 1) {
     idx = NZ - 1;

@@ -394,7 +394,7 @@ struct HaloProd {
   // spaced by (LOGM_MAX - LOGM_MIN) / NM
   __device__ static double minterp(const double* arr, double m) {
     double f = (log10(m) - LOGM_MIN) / (LOGM_MAX - LOGM_MIN) * (NM - 1);
-    int idx = (int)f;
+    int idx = f > 0 ? (int)f : 0;  // a mass below the table, or NaN: no index outside it
     f -= idx;
     if (idx >= NM - 1) {
       idx = NM - 2;
