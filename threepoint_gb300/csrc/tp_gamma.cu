@@ -343,7 +343,8 @@ struct GammaPolicy {
   };
   __device__ __forceinline__ bool geometry(double phi, double psi, Geo& G) const {
     double c, s;
-    if constexpr (sizeof(R) == 4) {  // 2^-60 absolute, on the integer pipe
+    if constexpr (sizeof(R) == 4) {  // on the integer pipe, for arguments in [0, 8)
+      if (!(psi >= 0 && psi < 8 && phi >= 0 && phi < 16)) return false;
       int64_t qs, qc;
       i64_sincos(psi, d_i64sin, qs, qc);
       G.sp = i64_q62(qs), G.cp = i64_q62(qc);
