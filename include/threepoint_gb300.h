@@ -446,6 +446,9 @@ int tp_mlp_train_step_device(tp_mlp* m, const float* x_dev, const float* t_dev, 
 /* waits for the network's stream; TP_ERR_CUDA if a kernel's tensor-core wait
  * reached its iteration limit */
 int tp_mlp_sync(tp_mlp* m);
+/* polls of a tensor-core wait before it gives up (< 0: the default). 0 lets
+ * every wait expire at once: how the error path is tested */
+int tp_mlp_set_wait_limit(tp_mlp* m, int iterations);
 void* tp_mlp_stream(const tp_mlp* m);
 /* C = A B^T on the tensor cores (device pointers, the network's stream): A
  * [M][lda], B [N][ldb] BF16 with K contiguous, C [M][ldc] FP32; M % 128 == 0,

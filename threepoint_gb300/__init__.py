@@ -212,6 +212,7 @@ def lib():
         L.tp_mlp_gradients.argtypes = [p, dp, dp, l, dp, dp]
         L.tp_mlp_train_step_device.argtypes = [p, p, p, l, C.c_float, p]
         L.tp_mlp_sync.argtypes = [p]
+        L.tp_mlp_set_wait_limit.argtypes = [p, i]
         L.tp_mlp_stream.argtypes = [p]
         L.tp_mlp_stream.restype = p
         L.tp_gemm_bf16_device.argtypes = [p, p, i, p, i, p, i, i, i, i]

@@ -73,15 +73,16 @@ struct GemmArgs {
   const float* b5;  // device scalar
   float* y;
   unsigned* err;  // bit 0: an mbarrier wait reached its limit
+  int spin;       // limit of the main loops' waits (the drain's is MBAR_SPIN)
 };
 
 // ---- tcgen05 / mbarrier primitives (inline PTX) -----------------------------
 __device__ __forceinline__ void mbar_init(uint32_t a, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint32_t a, uint32_t parity, int limit) {
   uint32_t ok = 0;
-  for (int it = 0; it < MBAR_SPIN && !ok; ++it)
+  for (int it = 0; it < limit && !ok; ++it)
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
@@ -355,10 +356,13 @@ __global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_rows(GemmArgs g) {
       for (int s = 0; s < nslab; ++s) mma_slab(tmem, m.a + s * GEMM_SLAB_A, m.b + s * GEMM_SLAB_B, idesc, s == 0);
       tc_commit(bar);
     }
-    ok = mbar_wait(bar, parity);
-    parity ^= 1;
+    ok = mbar_wait(bar, parity, g.spin);
     ok = __syncthreads_and(ok);
-    if (!ok) break;
+    if (!ok) {
+      mbar_wait(bar, parity, MBAR_SPIN);  // the tile's MMAs still read shared memory
+      break;
+    }
+    parity ^= 1;
     tc_fence_after();
     if (t + (int)gridDim.x < ntile) load_a(t + gridDim.x);
     gemm_epilogue(g, tmem, t * GEMM_BM);
@@ -387,6 +391,7 @@ __global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_ring(GemmArgs g) {
   };
   for (int s = 0; s < GEMM_STAGES - 1; ++s) load(s);
   bool ok = true;
+  int last = 0;  // the last slab whose MMAs are committed
   for (int s = 0; s < nslab; ++s) {
     load_wait<GEMM_STAGES - 2>();  // slab s has landed
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -397,16 +402,20 @@ __global__ void __launch_bounds__(GEMM_NT, 1) k_gemm_ring(GemmArgs g) {
       mma_slab(tmem, m.a + b * GEMM_SLAB_A, m.b + b * GEMM_SLAB_B, idesc, s == 0);
       tc_commit(smem_u32(&m.bars[b]));
     }
+    last = s;
     // slab s - 1's buffer is free once its MMAs are done: slab s + 3 goes there
     if (s > 0) {
-      ok = mbar_wait(smem_u32(&m.bars[(s - 1) % GEMM_STAGES]), ((s - 1) / GEMM_STAGES) & 1);
+      ok = mbar_wait(smem_u32(&m.bars[(s - 1) % GEMM_STAGES]), ((s - 1) / GEMM_STAGES) & 1, g.spin);
       ok = __syncthreads_and(ok);
       if (!ok) break;
     }
     load(s + GEMM_STAGES - 1);
   }
-  if (ok) ok = mbar_wait(smem_u32(&m.bars[(nslab - 1) % GEMM_STAGES]), ((nslab - 1) / GEMM_STAGES) & 1);
+  // MMAs complete in order: this wait covers all of them, after an expired one too
+  const uint32_t bar = smem_u32(&m.bars[last % GEMM_STAGES]), parity = (last / GEMM_STAGES) & 1;
+  if (ok) ok = mbar_wait(bar, parity, g.spin);
   ok = __syncthreads_and(ok);
+  if (!ok) mbar_wait(bar, parity, MBAR_SPIN);
   load_wait<0>();
   tc_fence_after();
   if (ok) gemm_epilogue(g, tmem, m0);
@@ -693,6 +702,7 @@ struct tp_mlp {
   double* lpart = nullptr;
   float* loss = nullptr;
   unsigned* d_err = nullptr;
+  int spin = MBAR_SPIN;  // limit of the GEMMs' waits
 };
 
 static int mlp_fail(tp_mlp* m, int st, const std::string& msg) {
@@ -724,6 +734,7 @@ static cudaError_t gemm(tp_mlp* m, GemmArgs a) {
     return cudaErrorInvalidValue;
   if (a.M > 0 && a.K <= 0) return cudaSuccess;  // nothing to sum
   a.err = m->d_err;
+  a.spin = m->spin;
   const int tiles = a.M / GEMM_BM;
   // B in shared memory while it fits; else (and for K slices) the slab ring
   if (a.kslices == 1 && a.K <= GEMM_KMAX)
@@ -1074,6 +1085,12 @@ extern "C" int tp_mlp_train_step_device(tp_mlp* m, const float* x_dev, const flo
 }
 
 // status of the asynchronous steps so far (synchronises the stream)
+extern "C" int tp_mlp_set_wait_limit(tp_mlp* m, int iterations) {
+  if (!m) return TP_ERR_ARG;
+  m->spin = iterations < 0 ? MBAR_SPIN : iterations;
+  return TP_OK;
+}
+
 extern "C" int tp_mlp_sync(tp_mlp* m) {
   if (!m) return TP_ERR_ARG;
   cudaSetDevice(m->device);
