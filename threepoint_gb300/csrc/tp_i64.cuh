@@ -5,16 +5,17 @@
 // log2 0.050, 1/x 0.35), so a 64-bit mantissa product made of three IMAD.WIDE
 // is about nine times cheaper than a DMUL. This header holds the pieces the
 // FP64 integrands are made of:
-//   Sf         a positive number m 2^e with a 64-bit mantissa (at least 58
-//              significant bits are kept between operations; the exponent has
-//              32 bits, so nothing in between overflows or underflows)
+//   Sf         a positive number m 2^e with a 64-bit mantissa (sums and products
+//              of mantissas with up to four leading zeros are within 2^-57; the
+//              exponent has 32 bits, so nothing in between overflows or underflows)
 //   Q52        a signed 64-bit fixed-point number in units of 2^-52: the
 //              base-2 exponents
 //   i64_exp2   2^x of a Q52 by a 256-entry table and a fifth-order polynomial
 //              (relative error below 2^-58)
 //   i64_log2   log2 of a 64-bit mantissa in Q57 by the same kind of table
 // Everything is plain integer arithmetic, the same on host and device, so the
-// error bounds are tested on the CPU.
+// error bounds are tested on the CPU; sf_rcp's start value alone differs (the
+// SFU's on the device), and its steps are tested with starts 2 ulp off.
 #pragma once
 #include <math.h>
 #include <stdint.h>
@@ -166,7 +167,8 @@ struct Sf {
 TP_HD Sf sf_mul(Sf a, Sf b) { return {i64_mulhi(a.m, b.m), a.e + b.e + 64}; }
 
 // the operand with the larger exponent keeps its unit (after one common shift
-// that makes room for the carry), the other is shifted to it
+// that makes room for the carry), the other is shifted to it; both lose less
+// than a unit of a result of 2^58 or more
 TP_HD Sf sf_add(Sf a, Sf b) {
   const int d = a.e - b.e;
   const int sa = (d < 0 ? -d : 0) + 1, sb = (d > 0 ? d : 0) + 1;
@@ -218,12 +220,23 @@ TP_HD double sf_to(Sf a) {
 #endif
 }
 
-// 1 / a: a start of 21 bits or more from the SFU and one third-order step,
-// y (1 + e + e^2) with e = 1 - m y
+// 1 / a: a start of 21 bits or more and one third-order step,
+// y (1 + e + e^2) with e = 1 - m y. a normalised, yu the start's float bits
+TP_HD Sf sf_rcp_step(Sf a, uint32_t yu) {
+  const uint32_t h = (uint32_t)(a.m >> 32);  // m: Q64 in [1/2, 1)
+  const uint32_t yq = yu >= 0x40000000u ? 0xffffff00u : 0x80000000u | (yu << 8);  // Q31 in [1, 2)
+  const uint64_t my = (uint64_t)h * yq + (((uint64_t)(uint32_t)a.m * yq) >> 32);  // Q63, near 1
+  const int64_t e = (int64_t)((1ull << 63) - my);                                 // |e| < 2^-20
+  const int32_t eh = (int32_t)(e >> 21);                                          // Q42
+  const int64_t s = e + (((int64_t)eh * eh) >> 21);                               // e + e^2, Q63
+  const int64_t c = ((int64_t)(int32_t)(s >> 32) * (int64_t)yq) + (int64_t)(((uint64_t)(uint32_t)s * yq) >> 32);
+  return {((uint64_t)yq << 31) + (uint64_t)c, -126 - a.e};  // y (1 + s) in Q62
+}
+// the float of m's upper bits, and 1 / a from its reciprocal
+TP_HD uint32_t sf_rcp_arg(Sf a) { return 0x3f000000u | (((uint32_t)(a.m >> 32) << 1) >> 9); }
 TP_HD Sf sf_rcp(Sf a) {
   a = sf_norm(a);
-  const uint32_t h = (uint32_t)(a.m >> 32);  // m: Q64 in [1/2, 1)
-  const uint32_t fu = 0x3f000000u | ((h << 1) >> 9);
+  const uint32_t fu = sf_rcp_arg(a);
 #if defined(__CUDA_ARCH__)
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(fu)));
@@ -235,13 +248,7 @@ TP_HD Sf sf_rcp(Sf a) {
   y = 1.0f / f;
   memcpy(&yu, &y, 4);
 #endif
-  const uint32_t yq = yu >= 0x40000000u ? 0xffffff00u : 0x80000000u | (yu << 8);  // Q31 in [1, 2)
-  const uint64_t my = (uint64_t)h * yq + (((uint64_t)(uint32_t)a.m * yq) >> 32);  // Q63, near 1
-  const int64_t e = (int64_t)((1ull << 63) - my);                                 // |e| < 2^-20
-  const int32_t eh = (int32_t)(e >> 21);                                          // Q42
-  const int64_t s = e + (((int64_t)eh * eh) >> 21);                               // e + e^2, Q63
-  const int64_t c = ((int64_t)(int32_t)(s >> 32) * (int64_t)yq) + (int64_t)(((uint64_t)(uint32_t)s * yq) >> 32);
-  return {((uint64_t)yq << 31) + (uint64_t)c, -126 - a.e};  // y (1 + s) in Q62
+  return sf_rcp_step(a, yu);
 }
 
 // ---- 2^x -----------------------------------------------------------------------
@@ -276,7 +283,8 @@ TP_HD int64_t i64_fix(double x) {
 }
 
 // ---- sine and cosine ---------------------------------------------------------------
-// of x in [0, 8), Q62 signed, within 2^-60 absolute: the quarter turn's 64
+// of x in [0, 8), Q62 signed, within 2^-57.6 absolute (two units of 2^-60 turns
+// of the argument; 2^-58.7 measured): the quarter turn's 64
 // cells by table, sin and cos of the distance d to a cell's centre
 // (|d| < pi/256) by their series to d^7 and d^6
 TP_HD void i64_sincos(double x, const uint64_t* __restrict__ tab, int64_t& sn, int64_t& cs) {
