@@ -93,7 +93,7 @@ struct PellProd {
   static constexpr int REC = (int)sizeof(Rec);
   const int* job_order = nullptr;
   static constexpr bool REF = sizeof(R) == 8;
-  int ref;
+  int ref, one;
   static constexpr size_t HC_BYTES = sizeof(R) * HC_COUNT * NNODE;
   static constexpr size_t PSMEM = HC_BYTES + (REF ? sizeof(PellShared64) : 0) + sizeof(CosmoK<R>) + 64;
 
@@ -140,6 +140,7 @@ struct PellProd {
       if constexpr (REF) {
         load64();
         __syncthreads();
+        one = !(ck.c64.ok && shared64().hi > 0);
       }
       loaded = 1;
     }
@@ -223,7 +224,7 @@ struct PellProd {
       }
     } else if (r.los) {
       const PellShared64& s = shared64();
-      bool in = ck.c64.ok && !ref;
+      bool in = !one && !ref;
       for (int i = 0; i < NL; ++i) in = in && ell[i] >= s.lo && ell[i] <= s.hi;
       r.f64form = !in;
       for (int i = 0; i < NL; ++i) {
@@ -317,7 +318,7 @@ struct BkProd {
   static constexpr int REC = (int)sizeof(Rec);
   const int* job_order = nullptr;
   static constexpr bool REF = sizeof(R) == 8;  // FP64 instructions beside the integer form
-  int ref;
+  int ref, one;
   static constexpr size_t NODE_BYTES = sizeof(R) == 4 ? sizeof(R) * NCP * NNODE : sizeof(Node64) * NNODE;
   static constexpr size_t EX2_BYTES = sizeof(R) == 4 ? 0 : sizeof(I64Tables::ex2);
   static constexpr size_t PSMEM = NODE_BYTES + EX2_BYTES + sizeof(CosmoK<R>) + 64;
@@ -339,6 +340,7 @@ struct BkProd {
       __syncthreads();
       const uint32_t* src = (const uint32_t*)(const void*)ncoef;
       if constexpr (sizeof(R) == 8) {
+        one = !ck.c64.ok;
         src = (const uint32_t*)(const void*)ck.n64;
         uint64_t* ex = (uint64_t*)(psmem + NODE_BYTES);
         for (int i = threadIdx.x; i < 256; i += blockDim.x) ex[i] = d_i64tab.ex2[i];
@@ -389,7 +391,7 @@ struct BkProd {
     (void)p;
     Rec& r = *(Rec*)recp;
     if constexpr (sizeof(R) == 8) {
-      if (ref || !ck.c64.ok) return setup_f64(x, th, lmax, r);
+      if (ref || one) return setup_f64(x, th, lmax, r);
     }
     double l1 = exp(x[0]), l2 = exp(x[1]), l5 = exp(x[2]), c1 = cos(x[3]), c2 = cos(x[4]);
     double l3 = sqrt(l1 * l1 + l2 * l2 + 2 * l1 * l2 * c1);

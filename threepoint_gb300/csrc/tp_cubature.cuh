@@ -395,7 +395,7 @@ __host__ __device__ constexpr size_t engine_smem_bytes() {
 template <int DIM, int FDIM, int NT, bool REF>
 __device__ __forceinline__ void engine_select(Slot<DIM, FDIM> S, EngineShared<FDIM>* es, EngineCfg cfg,
                                               unsigned long long* stage, int stage_bytes, int sweep, int npend,
-                                              int ref) {
+                                              int ref, bool ties) {
   constexpr int NP = GMRule<DIM>::NP;
   typedef unsigned long long u64;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -621,7 +621,8 @@ __device__ __forceinline__ void engine_select(Slot<DIM, FDIM> S, EngineShared<FD
 
   // ---------------- ties that the reference form decides --------------
   if constexpr (REF) {
-    if (!ref && tau != 0ull) {
+    // (a job that has the reference form alone has decided them already)
+    if (ties && !ref && tau != 0ull) {
       const double kt = __longlong_as_double((long long)tau);
       const double b0 = kt * (1.0 - TIE_REL), b1 = kt * (1.0 + TIE_REL);
       if (tid == 0) es->nband = es->nref = 0;
@@ -727,8 +728,8 @@ __device__ __forceinline__ void engine_select(Slot<DIM, FDIM> S, EngineShared<FD
 template <int DIM, int FDIM, int NT, bool REF>
 __device__ __noinline__ void engine_select_call(Slot<DIM, FDIM> S, EngineShared<FDIM>* es, EngineCfg cfg,
                                                 unsigned long long* stage, int stage_bytes, int sweep, int npend,
-                                                int ref) {
-  engine_select<DIM, FDIM, NT, REF>(S, es, cfg, stage, stage_bytes, sweep, npend, ref);
+                                                int ref, bool ties) {
+  engine_select<DIM, FDIM, NT, REF>(S, es, cfg, stage, stage_bytes, sweep, npend, ref, ties);
 }
 
 // ---------------------------------------------------------------------------
@@ -744,7 +745,8 @@ __device__ __noinline__ void engine_select_call(Slot<DIM, FDIM> S, EngineShared<
 //   static constexpr size_t PSMEM (policy shared bytes)
 //   static constexpr bool REF (optional): the policy has two forms of the
 //   integrand that agree to rounding, a fast one and the reference form
-//   (int ref: 0, or not for the reference form; set here). An integrand symmetric under an exchange or a
+//   (int ref: 0, or not for the reference form; set here; int one: set by
+//   begin_job where a job has the reference form alone). An integrand symmetric under an exchange or a
 //   reflection of its variables gives mirror-image regions whose errors differ
 //   only by rounding, and where a sweep's cut falls between them the reference
 //   form's rounding decides whether one or both are split (a bitwise tie splits
@@ -1026,9 +1028,10 @@ __device__ void adaptive_body(P& pol, int njobs, int* job_counter, const EngineC
       // pass, or a stop)
       if (crank == 0) {
         if constexpr (REF)
-          engine_select_call<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref);
+          engine_select_call<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref,
+                                              !pol.one);
         else
-          engine_select<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref);
+          engine_select<DIM, FDIM, NT, REF>(S, es, cfg, (unsigned long long*)recs, stage_bytes, sweep, npend, ref, false);
       }
       engine_cluster_sync<CS>();
       if (es0->stop) break;

@@ -163,7 +163,7 @@ struct GammaPolicy {
   // the set-up below and its reference form (the trigonometric one) decide
   // together where the cubature cuts between tied regions
   static constexpr bool REF = true;
-  int ref = 0;
+  int ref = 0, one = 0;
   // per job: sides and half interior angle of term j, its constant phase
   struct Term {
     double a, b, ch, sh, ce, se;
@@ -227,6 +227,10 @@ struct GammaPolicy {
         sincos(j == 0 ? p3 - p2 : j == 1 ? p3 - p1 - 2 * p2 : p1 - p2 + 2 * p3, &t.se, &t.ce);
       }
       s_term[j] = t;
+    }
+    if constexpr (sizeof(R) == 8) {
+      const CosmoK<double>& K = ck[cosmo];
+      one = !(K.c64.ok && K.n64[0].ok);
     }
     zmax = cosm[cosmo].zmax;
     xmin[0] = 0;
@@ -317,9 +321,9 @@ struct GammaPolicy {
     (void)p;
     Rec& r = *(Rec*)recp;
     if constexpr (sizeof(R) == 4) {
-      return ref ? setup_ref(x, r) : setup_f32(x, r);
+      return ref || one ? setup_ref(x, r) : setup_f32(x, r);
     } else {
-      r.f64form = ref || !setup_f64(x, r);
+      r.f64form = ref || one || !setup_f64(x, r);
       if (r.f64form) {
         const bool live = setup_ref(x, r.d);
         r.live = live;

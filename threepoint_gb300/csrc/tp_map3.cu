@@ -69,7 +69,7 @@ struct Map3Policy {
   typedef typename std::conditional<sizeof(R) == 4, RecF, RecD>::type Rec;
   const int* job_order;
   static constexpr bool REF = sizeof(R) == 8;  // FP64 instructions beside the integer form
-  int ref = 0;
+  int ref = 0, one = 0;
   static constexpr int REC = (int)sizeof(Rec);
   static constexpr int PD = 1;
   static constexpr int NS = 1;
@@ -165,6 +165,7 @@ struct Map3Policy {
     xmax[1] = lm;
     xmax[2] = phimax;
     scale = wscale[c];
+    if constexpr (REF) one = !s_ck->c64.ok;
     s_live = live_counter(psmem);
     if (threadIdx.x == 0) *s_live = 0ull;
     __syncthreads();
@@ -215,7 +216,7 @@ struct Map3Policy {
         trif_from_tri(t, r.tri);
       }
     } else {
-      if (ref || !s_ck->c64.ok) return setup_f64(x, th, r);
+      if (ref || one) return setup_f64(x, th, r);
       double l1 = x[0], l2 = x[1], phi = x[2];
       double s = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(phi);
       double l3 = s > 0 ? sqrt(s) : 0.0;
