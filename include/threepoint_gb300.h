@@ -376,6 +376,13 @@ int tp_ctx_set_halo_cluster(tp_ctx* ctx, int ctas);
  * always. Same results bit for bit. */
 int tp_ctx_set_map3_cluster(tp_ctx* ctx, int on);
 
+/* The integrands that have a fast form beside their reference form (FP64: 64-bit
+ * integer arithmetic beside FP64 instructions; FP32 Gamma: point geometry from
+ * complex products beside angles) are evaluated in the reference form alone when
+ * on; default 0. FP64 forms follow at the next tp_set_cosmologies. Both forms
+ * refine the same regions: the switch is there to check that. */
+int tp_ctx_set_reference_forms(tp_ctx* ctx, int on);
+
 /* Halo model of T5-T7 (cuda_version/halomodel.cu), built per cosmology on
  * first use.
  * tp_halo_tables: out[0..127] = sigma^2(m_i), out[128..255] = dsigma^2/dm(m_i)

@@ -188,6 +188,7 @@ def lib():
         L.tp_ctx_set_cov_tolerance.argtypes = [p, i, d]
         L.tp_ctx_set_halo_cluster.argtypes = [p, i]
         L.tp_ctx_set_map3_cluster.argtypes = [p, i]
+        L.tp_ctx_set_reference_forms.argtypes = [p, i]
         L.tp_cov_params_from_file.argtypes = [C.c_char_p, C.POINTER(_CovParams)]
         L.tp_gamma_config_from_file.argtypes = [C.c_char_p, C.POINTER(_GammaConfig)]
         L.tp_gamma_triangles.argtypes = [C.POINTER(_GammaConfig), dp, dp]
@@ -541,6 +542,11 @@ class Context:
         """<Map^3> batches with no more integrals than CTA slots: one 8-CTA
         cluster per integral (on) or one CTA (off); 2: clusters for every batch."""
         _check(self._h, lib().tp_ctx_set_map3_cluster(self._h, 2 if on == 2 else int(bool(on))))
+
+    def set_reference_forms(self, on=True):
+        """The integrands' reference forms alone (FP64 instructions; FP32 Gamma:
+        angles); the FP64 ones from the next set_cosmologies on."""
+        _check(self._h, lib().tp_ctx_set_reference_forms(self._h, int(bool(on))))
 
     def set_halo_cluster(self, ctas=16):
         """CTAs per T5/T6/T7 integral: 16 (a 16-CTA cluster where the batch

@@ -473,7 +473,7 @@ extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n,
     e = build_tables(ctx->d_cos, ctx->d_eh, ctx->d_nz, nz_stride, ctx->d_tab, ctx->d_ncoef64, ctx->d_ncoef32,
                      ctx->d_fcoef32, ctx->d_hcoef, ctx->d_hcoef32, ctx->d_wscale64, ctx->d_wscale32, (CosmoK<double>*)ctx->d_ck64,
                      (CosmoK<float>*)ctx->d_ck32, ctx->d_plt, ctx->d_ehg,
-                     ctx->d_n64, ctx->d_p64, n, s);
+                     ctx->d_n64, ctx->d_p64, !ctx->reference_forms, n, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return tp_cuda(ctx, e, "table build");
   return TP_OK;
@@ -596,6 +596,12 @@ extern "C" int tp_ctx_set_escalation(tp_ctx* ctx, int max_region_cap) {
 extern "C" int tp_ctx_set_map3_cluster(tp_ctx* ctx, int on) {
   if (!ctx || on < 0 || on > 2) return TP_ERR_ARG;
   ctx->map3_cluster = on;
+  return TP_OK;
+}
+
+extern "C" int tp_ctx_set_reference_forms(tp_ctx* ctx, int on) {
+  if (!ctx || on < 0 || on > 1) return TP_ERR_ARG;
+  ctx->reference_forms = on;
   return TP_OK;
 }
 

@@ -63,6 +63,8 @@ struct tp_ctx {
   // <Map^3> host calls with no more integrals than CTA slots run one 8-CTA
   // cluster per integral (0: always one CTA per integral)
   int map3_cluster = 1;
+  // the integrands' reference forms alone (tp_ctx_set_reference_forms)
+  int reference_forms = 0;
   // relative tolerance of the T5, T6, T7 integrals (index 5..7); 0 = the reference's
   double cov_rel_tol[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 

@@ -721,6 +721,7 @@ static int run_gamma(tp_ctx* ctx, int cosmo, const double* d_x, const int* d_com
   pol.cosm = ctx->d_cos;
   pol.ck = (const CosmoK<R>*)(sizeof(R) == 8 ? ctx->d_ck64 : ctx->d_ck32);
   pol.cosmo = cosmo;
+  pol.one = ctx->reference_forms;
   pol.out = d_out;
   pol.status = d_status;
   EngineCfg cfg{0.0, rel_tol, TP_NORM_L1, cap, 2000};
@@ -787,6 +788,7 @@ extern "C" int tp_gamma_integrand_points(tp_ctx* ctx, int cosmo_index, const dou
     pol.cosm = ctx->d_cos;
     pol.ck = (const CosmoK<double>*)ctx->d_ck64;
     pol.cosmo = cosmo_index;
+    pol.one = ctx->reference_forms;
     pol.out = nullptr;
     pol.status = nullptr;
     k_gamma_points<double><<<1, nt, GammaPolicy<double>::PSMEM, s>>>(pol, (const double*)(b + o_p), n,
@@ -800,6 +802,7 @@ extern "C" int tp_gamma_integrand_points(tp_ctx* ctx, int cosmo_index, const dou
     pol.cosm = ctx->d_cos;
     pol.ck = (const CosmoK<float>*)ctx->d_ck32;
     pol.cosmo = cosmo_index;
+    pol.one = ctx->reference_forms;
     pol.out = nullptr;
     pol.status = nullptr;
     k_gamma_points<float><<<1, nt, GammaPolicy<float>::PSMEM, s>>>(pol, (const double*)(b + o_p), n,
