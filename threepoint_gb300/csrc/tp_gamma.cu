@@ -428,8 +428,10 @@ struct GammaPolicy {
   }
   // the same for an absolute error of ulps units of 2^-53 |scale|
   static __device__ __forceinline__ bool rounds_alike(double v, double scale, int ulps) {
-    const int de = ((__double2hiint(scale) >> 20) & 2047) - ((__double2hiint(v) >> 20) & 2047) + 1;
-    return de < 20 && rounds_alike(v, de > 0 ? ulps << de : ulps);
+    // no value is further than 2^28 units from the middle: a larger bound is
+    // never met (and its shift would leave 32 bits)
+    const int de = max(0, ((__double2hiint(scale) >> 20) & 2047) - ((__double2hiint(v) >> 20) & 2047) + 1);
+    return de < 20 && ulps < (0x10000000 >> de) && rounds_alike(v, ulps << de);
   }
 
   __device__ bool setup_f32(const double* x, RecF& r) const {
@@ -444,7 +446,7 @@ struct GammaPolicy {
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const double A2 = G.A2[j], kap = G.k2[j] / A2;
-      same = same && kap < 1e3 && A2 > 1e-60 && A2 < 1e60;
+      same = same && kap < 1e3 && A2 > 1e-60 && A2 < 1e60 && G.mag[j] > 1e-30;  // (cre, cim normal floats)
       const int m = 128 + (int)(64 * fmin(kap, 1e3) + 16 * fmin(ib2, 1e4));
       const int64_t la = i64_log2(A2, d_i64tab) / 2;  // log2 A_j, Q57
       const double l2 = (double)la * 0x1p-57, ia = sf_to(i64_exp2(-(la >> 5), d_i64tab.ex2));
