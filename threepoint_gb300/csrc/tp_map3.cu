@@ -216,14 +216,17 @@ struct Map3Policy {
         trif_from_tri(t, r.tri);
       }
     } else {
-      if (ref || one) return setup_f64(x, th, r);
-      double l1 = x[0], l2 = x[1], phi = x[2];
-      double s = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(phi);
-      double l3 = s > 0 ? sqrt(s) : 0.0;
-      double outer = l1 * l2 * uhat(l1 * th[0]) * uhat(l2 * th[1]) * uhat(l3 * th[2]);
-      live = !(l1 == 0 || l2 == 0 || l3 == 0) && l1 > 1.0e-10 && l2 > 1.0e-10 && l3 > 1.0e-10 && outer != 0.0;
-      r.outer = live ? outer : 0.0;
-      if (live && !tri64_record(l1, l2, l3, *s_ck, r.tri)) setup_f64(x, th, r);
+      if (ref || one) {
+        live = setup_f64(x, th, r);
+      } else {
+        double l1 = x[0], l2 = x[1], phi = x[2];
+        double s = l1 * l1 + l2 * l2 + 2 * l1 * l2 * cos(phi);
+        double l3 = s > 0 ? sqrt(s) : 0.0;
+        double outer = l1 * l2 * uhat(l1 * th[0]) * uhat(l2 * th[1]) * uhat(l3 * th[2]);
+        live = !(l1 == 0 || l2 == 0 || l3 == 0) && l1 > 1.0e-10 && l2 > 1.0e-10 && l3 > 1.0e-10 && outer != 0.0;
+        r.outer = live ? outer : 0.0;
+        if (live && !tri64_record(l1, l2, l3, *s_ck, r.tri)) setup_f64(x, th, r);
+      }
     }
     if constexpr (sizeof(R) == 4) r.live = live;
     if (live && nlive && !ref) atomicAdd(s_live, 1ull);
