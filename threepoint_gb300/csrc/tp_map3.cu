@@ -378,20 +378,24 @@ __global__ void k_bkappa_points_f32(const int* cosmo_idx, const double* ell, lon
   if (lane == 0) out[w] = s * wscale[c];
 }
 
-// FP64: a block takes BK_PTS points; one thread a point sets its triangle up
-// in shared memory, then every thread sums the nodes of one (point, node
-// group) item, a warp's lanes at one group of neighbouring points, so that a
-// node row is one broadcast load.
-constexpr int BK_PTS = 32, BK_G = 8;
-__global__ void __launch_bounds__(BK_PTS* BK_G, 2)
+// FP64: a block takes PTS points; one thread a point sets its triangle up in
+// shared memory, then every thread evaluates the nodes of one (point, node
+// group) item, a warp's lanes at neighbouring points, so that a node row is a
+// broadcast load. PTS = 32: twelve nodes a thread. PTS = 8: three, for batches
+// that leave the SMs idle otherwise (BK_SMALL). The sums are those of eight
+// groups of twelve either way, so a point's value does not depend on its batch.
+constexpr int BK_NT = 256, BK_G = 8;
+template <int PTS>
+__global__ void __launch_bounds__(BK_NT, 2)
     k_bkappa_points_f64(const int* cosmo_idx, const double* ell, long n, const double* node_coef,
                         const double* wscale, const CosmoK<double>* ck, double* out) {
-  __shared__ Tri64 tri[BK_PTS];
+  constexpr int G = BK_NT / PTS, PER = NNODE / G;
+  __shared__ Tri64 tri[PTS];
   __shared__ uint64_t ex2[256];
-  __shared__ double part[BK_G][BK_PTS];
-  static_assert(BK_PTS * BK_G == 256, "the table load takes one entry a thread");
-  const int q = threadIdx.x % BK_PTS, g = threadIdx.x / BK_PTS;
-  const long p = (long)blockIdx.x * BK_PTS + q;
+  __shared__ double part[G == BK_G ? BK_G : NNODE][PTS];  // sums of a group, or every node
+  static_assert(BK_NT == 256 && NNODE % G == 0, "the table load takes one entry a thread");
+  const int q = threadIdx.x % PTS, g = threadIdx.x / PTS;
+  const long p = (long)blockIdx.x * PTS + q;
   ex2[threadIdx.x] = d_i64tab.ex2[threadIdx.x];
   bool live = p < n;
   int c = 0;
@@ -402,24 +406,31 @@ __global__ void __launch_bounds__(BK_PTS* BK_G, 2)
     if (g == 0 && live) tri64_record(l1, l2, l3, ck[c], tri[q]);
   }
   __syncthreads();
-  double v = 0.0;
+  constexpr int STEP = G == BK_G ? PER : 1;  // nodes added before they are stored
   if (live) {
     const CosmoK<double>& K = ck[c];
     const double* nc = node_coef + (size_t)c * NCP * NNODE;
     if (tri[q].ok) {
-      v = bkappa64_nodes(K.n64, nc, g * (NNODE / BK_G), NNODE / BK_G, tri[q], K, ex2);
+      for (int j = g * PER; j < (g + 1) * PER; j += STEP)
+        part[j / STEP][q] = bkappa64_nodes(K.n64, nc, j, STEP, tri[q], K, ex2);
     } else {
       Tri<double> T;
       make_tri<double>(ell[3 * p], ell[3 * p + 1], ell[3 * p + 2], T);
-      v = bkappa_nodes_f64(nc, g * (NNODE / BK_G), NNODE / BK_G, T, K);
+      for (int j = g * PER; j < (g + 1) * PER; j += STEP) part[j / STEP][q] = bkappa_nodes_f64(nc, j, STEP, T, K);
     }
   }
-  part[g][q] = v;
   __syncthreads();
   if (g == 0 && p < n) {
     double s = 0.0;
+    if (live) {
+#pragma unroll 1
+      for (int k = 0; k < BK_G; ++k) {
+        double v = 0.0;
 #pragma unroll
-    for (int k = 0; k < BK_G; ++k) s += part[k][q];
+        for (int i = 0; i < NNODE / BK_G / STEP; ++i) v += part[k * (NNODE / BK_G / STEP) + i][q];
+        s += v;
+      }
+    }
     out[p] = live ? s * wscale[c] : 0.0;
   }
 }
@@ -642,12 +653,22 @@ cudaError_t launch_map3(const Map3Launch& L, int grid, size_t smem, char* scratc
                                 : launch_map3_t<float>(L, grid, smem, scratch, st);
 }
 
+// Below BK_SMALL points eight a block, else 32. Host call in us, 8 / 32 a block:
+// integer form 56 / 97 (8 points), 74 / 103 (2048), 116 / 108 (4096), 168 / 148
+// (8191); FP64 instructions of a tabulated P(k) 151 / 417 (8), 268 / 430 (2048),
+// 501 / 436 (4096)
+constexpr long BK_SMALL = 3584;
+
 cudaError_t launch_bkappa_points(int precision, const int* cosmo_idx, const double* ell, long n, const void* ncoef,
                                  const double* wscale, const void* ck, double* out, cudaStream_t st) {
   const int bs = 256;
   if (precision == TP_FP64)
-    k_bkappa_points_f64<<<(unsigned)((n + BK_PTS - 1) / BK_PTS), BK_PTS * BK_G, 0, st>>>(
-        cosmo_idx, ell, n, (const double*)ncoef, wscale, (const CosmoK<double>*)ck, out);
+    if (n < BK_SMALL)
+      k_bkappa_points_f64<8><<<(unsigned)((n + 7) / 8), BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
+                                                                        (const CosmoK<double>*)ck, out);
+    else
+      k_bkappa_points_f64<32><<<(unsigned)((n + 31) / 32), BK_NT, 0, st>>>(
+          cosmo_idx, ell, n, (const double*)ncoef, wscale, (const CosmoK<double>*)ck, out);
   else
     k_bkappa_points_f32<<<(unsigned)((n * 32 + bs - 1) / bs), bs, 0, st>>>(
         cosmo_idx, ell, n, (const float*)ncoef, wscale, (const CosmoK<float>*)ck, out);
