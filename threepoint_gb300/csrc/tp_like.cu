@@ -112,9 +112,20 @@ __global__ void __launch_bounds__(CNT) k_chi2(const double* xt, const double* da
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     double z = 0.0;
+    int k0 = 0;
 #pragma unroll 16
-    for (int k = 0; k <= i; ++k) z += xt[(size_t)k * n + i] * r[k];
-    acc += z * z;
+    for (; k0 < (i & ~31); ++k0) z = fma(xt[(size_t)k0 * n + i], r[k0], z);
+    // a warp's rows end in the same block of 32: its loads go out together
+    // (past the diagonal they are not used)
+    for (int h = 0; h < 2; ++h, k0 += 16) {
+      double a[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) a[u] = xt[(size_t)min(k0 + u, n - 1) * n + i];
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (k0 + u <= i) z = fma(a[u], r[k0 + u], z);
+    }
+    acc = fma(z, z, acc);
   }
   part[threadIdx.x] = acc;
   __syncthreads();
