@@ -310,9 +310,11 @@ static __device__ __noinline__ void f2_trees(double l1, double l2, double l3, do
 
 // false (T.ok = 0) where the triangle or the cosmology is outside its domain
 __device__ __forceinline__ bool tri64_record(double l1, double l2, double l3, const CosmoK<double>& K, Tri64& T) {
+  T.ok = 0;
+  if (!K.c64.ok) return false;
   double f2t[3];
   f2_trees(l1, l2, l3, f2t);
-  const bool ok = K.c64.ok && tri64_make(l1, l2, l3, f2t, K.c64.lo, K.c64.hi, d_i64tab, T);
+  const bool ok = tri64_make(l1, l2, l3, f2t, K.c64.lo, K.c64.hi, d_i64tab, T);
   T.ok = ok;
   return ok;
 }

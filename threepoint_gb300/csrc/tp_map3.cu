@@ -379,22 +379,24 @@ __global__ void k_bkappa_points_f32(const int* cosmo_idx, const double* ell, lon
 }
 
 // FP64: a block takes PTS points; one thread a point sets its triangle up in
-// shared memory, then every thread evaluates the nodes of one (point, node
-// group) item, a warp's lanes at neighbouring points, so that a node row is a
-// broadcast load. PTS = 32: twelve nodes a thread. PTS = 8: three, for batches
-// that leave the SMs idle otherwise (BK_SMALL). The sums are those of eight
-// groups of twelve either way, so a point's value does not depend on its batch.
+// shared memory. PTS = 32: every thread sums the twelve nodes of a group, a
+// warp's lanes at neighbouring points, so that a node row is a broadcast load.
+// PTS = 8, for batches that leave the SMs idle otherwise (BK_SMALL): three nodes
+// a thread, the lanes as above or (WARP, below eight points) a warp a point. The
+// sums are those of eight groups of twelve always, so a point's value does not
+// depend on its batch.
 constexpr int BK_NT = 256, BK_G = 8;
-template <int PTS>
+template <int PTS, bool WARP>
 __global__ void __launch_bounds__(BK_NT, 2)
     k_bkappa_points_f64(const int* cosmo_idx, const double* ell, long n, const double* node_coef,
                         const double* wscale, const CosmoK<double>* ck, double* out) {
   constexpr int G = BK_NT / PTS, PER = NNODE / G;
   __shared__ Tri64 tri[PTS];
   __shared__ uint64_t ex2[256];
-  __shared__ double part[G == BK_G ? BK_G : NNODE][PTS];  // sums of a group, or every node
+  constexpr int STEP = G == BK_G ? PER : 1;  // nodes added before they are stored
+  __shared__ double part[NNODE / STEP][PTS + (STEP == 1)];
   static_assert(BK_NT == 256 && NNODE % G == 0, "the table load takes one entry a thread");
-  const int q = threadIdx.x % PTS, g = threadIdx.x / PTS;
+  const int q = WARP ? threadIdx.x / G : threadIdx.x % PTS, g = WARP ? threadIdx.x % G : threadIdx.x / PTS;
   const long p = (long)blockIdx.x * PTS + q;
   ex2[threadIdx.x] = d_i64tab.ex2[threadIdx.x];
   bool live = p < n;
@@ -406,17 +408,16 @@ __global__ void __launch_bounds__(BK_NT, 2)
     if (g == 0 && live) tri64_record(l1, l2, l3, ck[c], tri[q]);
   }
   __syncthreads();
-  constexpr int STEP = G == BK_G ? PER : 1;  // nodes added before they are stored
   if (live) {
     const CosmoK<double>& K = ck[c];
     const double* nc = node_coef + (size_t)c * NCP * NNODE;
     if (tri[q].ok) {
-      for (int j = g * PER; j < (g + 1) * PER; j += STEP)
-        part[j / STEP][q] = bkappa64_nodes(K.n64, nc, j, STEP, tri[q], K, ex2);
+      for (int i = 0; i < PER / STEP; ++i)
+        part[g + i * G][q] = bkappa64_nodes(K.n64, nc, (g + i * G) * STEP, STEP, tri[q], K, ex2);
     } else {
       Tri<double> T;
       make_tri<double>(ell[3 * p], ell[3 * p + 1], ell[3 * p + 2], T);
-      for (int j = g * PER; j < (g + 1) * PER; j += STEP) part[j / STEP][q] = bkappa_nodes_f64(nc, j, STEP, T, K);
+      for (int i = 0; i < PER / STEP; ++i) part[g + i * G][q] = bkappa_nodes_f64(nc, (g + i * G) * STEP, STEP, T, K);
     }
   }
   __syncthreads();
@@ -654,20 +655,23 @@ cudaError_t launch_map3(const Map3Launch& L, int grid, size_t smem, char* scratc
 }
 
 // Below BK_SMALL points eight a block, else 32. Host call in us, 8 / 32 a block:
-// integer form 56 / 97 (8 points), 74 / 103 (2048), 116 / 108 (4096), 168 / 148
-// (8191); FP64 instructions of a tabulated P(k) 151 / 417 (8), 268 / 430 (2048),
-// 501 / 436 (4096)
+// integer form 57 / 97 (8 points), 73 / 102 (2048), 113 / 107 (4096); FP64
+// instructions of a tabulated P(k) 150 / 415 (8), 268 / 428 (2048), 501 / 434
+// (4096). A warp a point: 91 us of FP64 instructions for one point, 155 else.
 constexpr long BK_SMALL = 3584;
 
 cudaError_t launch_bkappa_points(int precision, const int* cosmo_idx, const double* ell, long n, const void* ncoef,
                                  const double* wscale, const void* ck, double* out, cudaStream_t st) {
   const int bs = 256;
   if (precision == TP_FP64)
-    if (n < BK_SMALL)
-      k_bkappa_points_f64<8><<<(unsigned)((n + 7) / 8), BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
+    if (n < 8)
+      k_bkappa_points_f64<8, true><<<1, BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
+                                                        (const CosmoK<double>*)ck, out);
+    else if (n < BK_SMALL)
+      k_bkappa_points_f64<8, false><<<(unsigned)((n + 7) / 8), BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
                                                                         (const CosmoK<double>*)ck, out);
     else
-      k_bkappa_points_f64<32><<<(unsigned)((n + 31) / 32), BK_NT, 0, st>>>(
+      k_bkappa_points_f64<32, false><<<(unsigned)((n + 31) / 32), BK_NT, 0, st>>>(
           cosmo_idx, ell, n, (const double*)ncoef, wscale, (const CosmoK<double>*)ck, out);
   else
     k_bkappa_points_f32<<<(unsigned)((n * 32 + bs - 1) / bs), bs, 0, st>>>(
