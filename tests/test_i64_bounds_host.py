@@ -25,3 +25,8 @@ def report(tmp_path_factory):
 @pytest.mark.parametrize("name,bound", [("add", 2.0 ** -57), ("sincos", 2.0 ** -57.6), ("rcp", 2.0 ** -60)])
 def test_bounds(report, name, bound):
     assert report[name] <= bound, (name, report[name])
+
+
+def test_rounding_claims(report):
+    assert report["alike"] > 100000
+    assert report["unlike"] == 0

@@ -420,28 +420,17 @@ struct GammaPolicy {
   // The FP32 record rounds the geometry's doubles. Where a value lies so near
   // the middle of two floats that the rounding error of this geometry or of
   // the reference form's (which grows with the cancellation in A_j and betabar)
-  // could reach it, the point takes the reference form, so that both make the
-  // same floats: ~1 point in 3000. ulps: that error in units of 2^-53 of v.
-  static __device__ __forceinline__ bool rounds_alike(double v, int ulps) {
-    const int low = __double2loint(v) & 0x1fffffff, d = low - 0x10000000;
-    return (d < 0 ? -d : d) > ulps;
-  }
-  // the same for an absolute error of ulps units of 2^-53 |scale|
-  static __device__ __forceinline__ bool rounds_alike(double v, double scale, int ulps) {
-    // no value is further than 2^28 units from the middle: a larger bound is
-    // never met (and its shift would leave 32 bits)
-    const int de = max(0, ((__double2hiint(scale) >> 20) & 2047) - ((__double2hiint(v) >> 20) & 2047) + 1);
-    return de < 20 && ulps < (0x10000000 >> de) && rounds_alike(v, ulps << de);
-  }
-
+  // could reach it (i64_rounds_alike with that error in units of 2^-53), the
+  // point takes the reference form, so that both make the same floats: ~1 point
+  // in 3000.
   __device__ bool setup_f32(const double* x, RecF& r) const {
     Geo G;
     r.live = zrow_f32(tab[cosmo], cosm[cosmo], x[0], r.nf);
     if (!r.live) return false;
     if (!geometry(x[1], x[2], G)) return setup_ref(x, r);
     const double ib2 = 1 / G.b2;
-    bool same = ib2 < 1e4 && rounds_alike(G.cp, 1.0, 64) && rounds_alike(G.sp, 1.0, 64) &&
-                rounds_alike(G.cph, 1.0, 64) && rounds_alike(G.b3, 64 + (int)(16 * ib2));
+    bool same = ib2 < 1e4 && i64_rounds_alike(G.cp, 1.0, 64) && i64_rounds_alike(G.sp, 1.0, 64) &&
+                i64_rounds_alike(G.cph, 1.0, 64) && i64_rounds_alike(G.b3, 64 + (int)(16 * ib2));
     r.bmin = (float)fmin(G.cp, fmin(G.sp, G.b3));
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
@@ -450,8 +439,8 @@ struct GammaPolicy {
       const int m = 128 + (int)(64 * fmin(kap, 1e3) + 16 * fmin(ib2, 1e4));
       const int64_t la = i64_log2(A2, d_i64tab) / 2;  // log2 A_j, Q57
       const double l2 = (double)la * 0x1p-57, ia = sf_to(i64_exp2(-(la >> 5), d_i64tab.ex2));
-      same = same && rounds_alike(ia, m) && rounds_alike(l2, 2.0, m) && rounds_alike(G.cre[j], G.mag[j], m) &&
-             rounds_alike(G.cim[j], G.mag[j], m);
+      same = same && i64_rounds_alike(ia, m) && i64_rounds_alike(l2, 2.0, m) && i64_rounds_alike(G.cre[j], G.mag[j], m) &&
+             i64_rounds_alike(G.cim[j], G.mag[j], m);
       r.invA[j] = (float)ia;
       r.l2A[j] = (float)l2;
       r.cre[j] = (float)G.cre[j];

@@ -311,6 +311,30 @@ TP_HD void i64_sincos(double x, const uint64_t* __restrict__ tab, int64_t& sn, i
 // Q62 to double
 TP_HD double i64_q62(int64_t q) { return (double)q * 0x1p-62; }
 
+// ---- rounding of a double to float ------------------------------------------------
+// whether every number within ulps units of 2^-52 2^floor(log2 |v|) of v rounds
+// to the same float (v a normal float's range)
+TP_HD uint64_t i64_bits(double x) {
+#if defined(__CUDA_ARCH__)
+  return (uint64_t)__double_as_longlong(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return u;
+#endif
+}
+TP_HD bool i64_rounds_alike(double v, int ulps) {
+  const int low = (int)((uint32_t)i64_bits(v) & 0x1fffffffu), d = low - 0x10000000;
+  return (d < 0 ? -d : d) > ulps;
+}
+// the same for an absolute error of ulps units of 2^-53 2^floor(log2 |scale|):
+// no value is further than 2^28 units from the middle of two floats, so a larger
+// bound is never met (and its shift would leave 32 bits)
+TP_HD bool i64_rounds_alike(double v, double scale, int ulps) {
+  const int e = (int)(i64_bits(scale) >> 52 & 2047) - (int)(i64_bits(v) >> 52 & 2047) + 1, de = e > 0 ? e : 0;
+  return de < 20 && ulps < (0x10000000 >> de) && i64_rounds_alike(v, ulps << de);
+}
+
 // ---- log2 -----------------------------------------------------------------------
 // log2 of a normalised mantissa m in [1, 2) (Q63): -log2 c + log2(1 + t) with
 // t = m c - 1 and c the table's reciprocal of m's 1/256-wide cell; Q62, within 2^-57
