@@ -320,6 +320,8 @@ void tp_ctx::free_cosmo() {
   d_ehg = nullptr;
   d_n64 = nullptr;
   d_p64 = nullptr;
+  i64_cap = 0;
+  i64_ready = 0;
   n_cosmo = 0;
   cosmo_cap = 0;
   nz_cap = 0;
@@ -392,6 +394,12 @@ extern "C" int tp_ctx_destroy(tp_ctx* c) {
   return TP_OK;
 }
 
+// Sets of up to this many cosmologies are built with the integer-arithmetic
+// tables of the FP64 integrands (382 KB a cosmology, 1.6% of the build's time);
+// larger ones when a first FP64 call asks for them, so that a batch in FP32 does
+// not pay for them (4096 cosmologies: 2.83 -> 1.34 GB, 3188 -> 3138 ms).
+static const int I64_EAGER = 24;
+
 extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n, const double* nz, int nz_stride,
                                   const double* pk, double dk, double kmin, double kmax) {
   TpRange nvtx_range("tp_set_cosmologies: table build");
@@ -450,8 +458,6 @@ extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n,
     if (e == cudaSuccess) e = dalloc((CosmoK<float>**)&ctx->d_ck32, cap);
     if (e == cudaSuccess) e = dalloc(&ctx->d_plt, (size_t)cap * PLT_N);
     if (e == cudaSuccess) e = dalloc(&ctx->d_ehg, (size_t)cap * EHG_N);
-    if (e == cudaSuccess) e = dalloc(&ctx->d_n64, (size_t)cap * NNODE);
-    if (e == cudaSuccess) e = dalloc(&ctx->d_p64, (size_t)cap * P64_N);
     if (e != cudaSuccess) {
       ctx->free_cosmo();
       return tp_cuda(ctx, e, "cosmology allocation");
@@ -472,10 +478,51 @@ extern "C" int tp_set_cosmologies(tp_ctx* ctx, const tp_cosmology* cosmo, int n,
   if (e == cudaSuccess)
     e = build_tables(ctx->d_cos, ctx->d_eh, ctx->d_nz, nz_stride, ctx->d_tab, ctx->d_ncoef64, ctx->d_ncoef32,
                      ctx->d_fcoef32, ctx->d_hcoef, ctx->d_hcoef32, ctx->d_wscale64, ctx->d_wscale32, (CosmoK<double>*)ctx->d_ck64,
-                     (CosmoK<float>*)ctx->d_ck32, ctx->d_plt, ctx->d_ehg,
-                     ctx->d_n64, ctx->d_p64, !ctx->reference_forms, n, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                     (CosmoK<float>*)ctx->d_ck32, ctx->d_plt, ctx->d_ehg, n, s);
   if (e != cudaSuccess) return tp_cuda(ctx, e, "table build");
+  ctx->pk_given = pk != nullptr;
+  ctx->i64_ready = 0;
+  if (ctx->i64_used || n <= I64_EAGER) {
+    const int st = ctx->ensure_i64();
+    if (st) return st;
+  }
+  e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return tp_cuda(ctx, e, "table build");
+  return TP_OK;
+}
+
+int tp_ctx::ensure_i64() {
+  if (i64_ready) return TP_OK;
+  // a tabulated P(k) has the FP64 instructions alone
+  if (pk_given || reference_forms) {
+    i64_ready = 1;
+    return TP_OK;
+  }
+  // no allocation under capture, and nothing recorded that a later call would
+  // rely on: those integrals run in FP64 instructions
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(stream, &cap);
+  if (e != cudaSuccess) return tp_cuda(this, e, "capture status");
+  if (cap != cudaStreamCaptureStatusNone) return TP_OK;
+  if (i64_cap < n_cosmo) {
+    cudaFree(d_n64);
+    cudaFree(d_p64);
+    d_n64 = nullptr;
+    d_p64 = nullptr;
+    i64_cap = 0;
+    const size_t m = std::max(n_cosmo, cosmo_cap);
+    e = dalloc(&d_n64, m * NNODE);
+    if (e == cudaSuccess) e = dalloc(&d_p64, m * P64_N);
+    if (e != cudaSuccess) {
+      cudaFree(d_n64);
+      d_n64 = nullptr;
+      return tp_cuda(this, e, "FP64 table allocation");
+    }
+    i64_cap = (int)m;
+  }
+  e = build_tables_i64(d_cos, d_eh, d_ncoef64, (CosmoK<double>*)d_ck64, d_n64, d_p64, n_cosmo, stream);
+  if (e != cudaSuccess) return tp_cuda(this, e, "FP64 table build");
+  i64_ready = i64_used = 1;
   return TP_OK;
 }
 
@@ -532,6 +579,7 @@ extern "C" int tp_bkappa_batch(tp_ctx* ctx, const int* cosmo_index, const double
   size_t b_ell = sizeof(double) * 3 * n, b_out = sizeof(double) * n, b_idx = cosmo_index ? sizeof(int) * n : 0;
   size_t off_out = (b_ell + 255) & ~size_t(255), off_idx = (off_out + b_out + 255) & ~size_t(255);
   int st = ctx->ensure_io(off_idx + b_idx + 256);
+  if (st == TP_OK && precision == TP_FP64) st = ctx->ensure_i64();
   if (st) return st;
   char* base = ctx->d_io;
   cudaStream_t s = ctx->stream;
@@ -558,6 +606,7 @@ extern "C" int tp_bkappa_nodes(tp_ctx* ctx, int cosmo_index, const double* ell, 
   const size_t b_ell = sizeof(double) * 3 * n, b_node = sizeof(double) * NNODE * n;
   const size_t o_t = (b_ell + 255) & ~size_t(255), o_b = o_t + ((b_node + 255) & ~size_t(255));
   int st = ctx->ensure_io(o_b + b_node + 256);
+  if (st == TP_OK && precision == TP_FP64) st = ctx->ensure_i64();
   if (st) return st;
   char* base = ctx->d_io;
   cudaStream_t s = ctx->stream;
@@ -622,6 +671,7 @@ extern "C" int tp_map3_jobs_device(tp_ctx* ctx, const int* job_cosmo, const doub
                             &smem, &scratch);
   if (e != cudaSuccess) return tp_cuda(ctx, e, "map3 plan");
   int st = ctx->ensure_scratch(scratch);
+  if (st == TP_OK && precision == TP_FP64) st = ctx->ensure_i64();
   if (st) return st;
   Map3Launch L;
   L.precision = precision;

@@ -51,8 +51,12 @@ struct tp_ctx {
   void* d_ck32 = nullptr;
   float4* d_plt = nullptr;  // [n_cosmo][PLT_N] log2 P_lin cubic segments
   // integer-arithmetic forms of the FP64 integrands (tp_bispec64.cuh)
-  tp::Node64* d_n64 = nullptr;   // [n_cosmo][NNODE]
-  tp::P64Cell* d_p64 = nullptr;  // [n_cosmo][P64_N]
+  tp::Node64* d_n64 = nullptr;   // [i64_cap][NNODE]
+  tp::P64Cell* d_p64 = nullptr;  // [i64_cap][P64_N]
+  int i64_cap = 0;
+  int i64_used = 0;   // an FP64 call has asked for them: sets are built with them from then on
+  int i64_ready = 0;  // built for the current cosmologies
+  int pk_given = 0;   // of the current cosmologies
   double* d_ehg = nullptr;  // [n_cosmo][EHG_N] 2 ln T(k) of the sigma(R) integrand
   // halo-model tables (covariance terms T5-T7), built per cosmology on first use
   tp::HaloTab* d_halo = nullptr;
@@ -86,6 +90,8 @@ struct tp_ctx {
   unsigned* d_diag = nullptr;
 
   void free_cosmo();
+  // the integer-arithmetic tables of the current cosmologies, if they are not there yet
+  int ensure_i64();
   int ensure_scratch(size_t bytes);
   int ensure_io(size_t bytes);
 };

@@ -345,7 +345,8 @@ struct BkProd {
         uint64_t* ex = (uint64_t*)(psmem + NODE_BYTES);
         for (int i = threadIdx.x; i < 256; i += blockDim.x) ex[i] = d_i64tab.ex2[i];
       }
-      for (int i = threadIdx.x; i < (int)(NODE_BYTES / 4); i += blockDim.x) ((uint32_t*)psmem)[i] = src[i];
+      if (src)  // (none for a cosmology without the integer form)
+        for (int i = threadIdx.x; i < (int)(NODE_BYTES / 4); i += blockDim.x) ((uint32_t*)psmem)[i] = src[i];
       __syncthreads();
       loaded = 1;
     }
@@ -643,6 +644,10 @@ static int run_pell_kind(tp_ctx* ctx, int cosmo, const JobSet& js, double theta_
                          double norm, double rel_tol, std::vector<double>& res, int& bad) {
   res.assign(js.jobs.size(), 0.0);
   if (js.jobs.empty()) return TP_OK;
+  if constexpr (sizeof(R) == 8) {
+    const int st = ctx->ensure_i64();
+    if (st) return st;
+  }
   PellProd<R, DIM, KIND> pol;
   memset(&pol, 0, sizeof(pol));
   pol.hcoef = (sizeof(R) == 8 ? (const R*)(const void*)ctx->d_hcoef : (const R*)(const void*)ctx->d_hcoef32) +
@@ -665,6 +670,10 @@ template <typename R>
 static int run_t4(tp_ctx* ctx, int cosmo, const JobSet& js, double norm, std::vector<double>& res, int& bad) {
   res.assign(js.jobs.size(), 0.0);
   if (js.jobs.empty()) return TP_OK;
+  if constexpr (sizeof(R) == 8) {
+    const int st = ctx->ensure_i64();
+    if (st) return st;
+  }
   BkProd<R> pol;
   memset(&pol, 0, sizeof(pol));
   pol.ncoef = (sizeof(R) == 8 ? (const R*)(const void*)ctx->d_ncoef64 : (const R*)(const void*)ctx->d_fcoef32) +

@@ -759,6 +759,10 @@ extern "C" int tp_gamma_integrand_points(tp_ctx* ctx, int cosmo_index, const dou
   cudaSetDevice(ctx->device);
   cudaError_t e = gamma_upload_constants();
   if (e != cudaSuccess) return tp_cuda(ctx, e, "ogata constants");
+  if (precision == TP_FP64) {
+    const int st64 = ctx->ensure_i64();
+    if (st64) return st64;
+  }
   const int jc[2] = {which, 0};  // job 0: component `which` of triangle 0
   const size_t o_c = 256, o_p = 512, o_o = o_p + ((sizeof(double) * 3 * n + 255) & ~size_t(255));
   int st = ctx->ensure_io(o_o + sizeof(double) * 2 * n + 256);
@@ -872,6 +876,10 @@ extern "C" int tp_gamma_batch(tp_ctx* ctx, int cosmo_index, const double* x, int
   cudaSetDevice(ctx->device);
   cudaError_t e = gamma_upload_constants();
   if (e != cudaSuccess) return tp_cuda(ctx, e, "ogata constants");
+  if (precision == TP_FP64) {
+    const int st64 = ctx->ensure_i64();
+    if (st64) return st64;
+  }
   std::vector<int> hst(n);
   int st = gamma_pass(ctx, cosmo_index, x, n, comp_mask, rel_tol, precision, ctx->region_cap, ctx->max_ctas, out,
                       hst.data());

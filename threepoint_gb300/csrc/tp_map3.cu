@@ -126,8 +126,9 @@ struct Map3Policy {
       constexpr int nbytes = (int)NODE_BYTES;
       static_assert(nbytes % 16 == 0, "bulk copy size must be a multiple of 16 bytes");
       if (threadIdx.x == 0) {
-        // the node table (10-20 KB) is staged by one bulk async copy
-        if (!bulk_copy_g2s(bar(psmem), psmem, src, nbytes)) {
+        // the node table (10-20 KB) is staged by one bulk async copy (none for
+        // a cosmology without the integer form's)
+        if (src && !bulk_copy_g2s(bar(psmem), psmem, src, nbytes)) {
           for (int i = 0; i < nbytes / 4; ++i) ((uint32_t*)psmem)[i] = ((const uint32_t*)src)[i];
         }
         *s_ck = ck[c];

@@ -904,7 +904,7 @@ TP_TABLE_KERNEL k_p64(const CosmoDev* cos, const EHConst* eh, P64Cell* p64, Cosm
 // cosmology takes that form when its P(k) is the fit's, its constants are
 // ordinary numbers and some ell range keeps every node inside the P table
 TP_TABLE_KERNEL k_node64(const CosmoDev* cos, const EHConst* eh, const double* ncoef, const P64Cell* p64, Node64* n64,
-                         CosmoK<double>* ck64, bool allow, int n) {
+                         CosmoK<double>* ck64, int n) {
   const int ci = blockIdx.x;
   if (ci >= n) return;
   double lo = 0x1p-36, hi = 0x1p26;
@@ -929,7 +929,7 @@ TP_TABLE_KERNEL k_node64(const CosmoDev* cos, const EHConst* eh, const double* n
     CosmoK<double>& k = ck64[ci];
     k.n64 = n64 + (size_t)ci * NNODE;
     k.c64.p = p64 + (size_t)ci * P64_N;
-    k.c64.ok = allow && !k.c64.bad && !cos[ci].pk_given && amax >= 0 && fabs(e.ns) < 3 && sf_ok(e.ehc) && sf_ok(e.omh2) && sf_ok(e.sa) &&
+    k.c64.ok = !k.c64.bad && !cos[ci].pk_given && amax >= 0 && fabs(e.ns) < 3 && sf_ok(e.ehc) && sf_ok(e.omh2) && sf_ok(e.sa) &&
                e.one_m_sa > -0.5 * e.sa && sf_ok(e.theta2) && e.c184 > 1e-6 && e.c184 < 1e6 && e.sh > 1e-3 &&
                e.sh < 1e6 && e.omh2 > 1e-6 && e.omh2 < 1e6 && lo < hi;
     k.c64.amax = k.c64.ok ? (uint64_t)i64_fix<59>(amax) : 0;
@@ -950,7 +950,7 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
                          double* d_ncoef, float* d_ncoef_f, float* d_fcoef_f, double* d_hcoef, float* d_hcoef_f,
                          double* d_wscale64,
                          double* d_wscale32, CosmoK<double>* d_ck64, CosmoK<float>* d_ck32, float4* d_plt,
-                         double* d_ehg, Node64* d_n64, P64Cell* d_p64, bool allow_i64, int n, cudaStream_t s) {
+                         double* d_ehg, int n, cudaStream_t s) {
   // every launch is made of one-warp blocks (see above). An SM runs blocks of
   // different kernels together only in one shared-memory/L1 configuration:
   // these kernels ask for the one k_map3 runs in (maximum shared memory).
@@ -1000,8 +1000,13 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
   k_finish<<<n, 32, 0, s>>>(d_cos, d_eh, d_tab, d_ncoef, d_ncoef_f, d_fcoef_f, d_wscale64, d_wscale32, d_ck64, d_ck32,
                             n);
   k_plin_table<<<n * (PLT_N / 128), 32, 0, s>>>(d_cos, d_eh, d_plt, d_ck32, n);
+  return cudaGetLastError();
+}
+
+cudaError_t build_tables_i64(const CosmoDev* d_cos, const EHConst* d_eh, const double* d_ncoef, CosmoK<double>* d_ck64,
+                             Node64* d_n64, P64Cell* d_p64, int n, cudaStream_t s) {
   k_p64<<<(unsigned)((long)n * P64_N / 32), 32, 0, s>>>(d_cos, d_eh, d_p64, d_ck64, n);
-  k_node64<<<n, 32, 0, s>>>(d_cos, d_eh, d_ncoef, d_p64, d_n64, d_ck64, allow_i64, n);
+  k_node64<<<n, 32, 0, s>>>(d_cos, d_eh, d_ncoef, d_p64, d_n64, d_ck64, n);
   return cudaGetLastError();
 }
 

@@ -16,7 +16,12 @@ cudaError_t build_tables(const CosmoDev* d_cos, EHConst* d_eh, const double* d_n
                          double* d_ncoef, float* d_ncoef_f, float* d_fcoef_f, double* d_hcoef, float* d_hcoef_f,
                          double* d_wscale64,
                          double* d_wscale32, CosmoK<double>* d_ck64, CosmoK<float>* d_ck32, float4* d_plt,
-                         double* d_ehg, Node64* d_n64, P64Cell* d_p64, bool allow_i64, int n, cudaStream_t s);
+                         double* d_ehg, int n, cudaStream_t s);
+
+// Node rows and P(k) tables of the integer-arithmetic FP64 integrands, and
+// ck64's c64 that switches that form on (after build_tables).
+cudaError_t build_tables_i64(const CosmoDev* d_cos, const EHConst* d_eh, const double* d_ncoef, CosmoK<double>* d_ck64,
+                             Node64* d_n64, P64Cell* d_p64, int n, cudaStream_t s);
 
 // Fills the node rows (HN_*) of the halo-model tables of cosmology ci on
 // stream s from its z-tables (launches one small kernel).
