@@ -15,7 +15,7 @@ three steps:
    constants the reference's copyConstants / set_cosmology /
    compute_weights_bessel upload (bispectrum.cu:90-219, gamma.cu:13-56), runs
    the harness kernels and writes the outputs (default
-   gpurun_out/ref_device_out.npz).
+   oracle/_ref/ref_device_out.npz).
 3. ``finish``: merges inputs and outputs into tests/golden/reference_device.npz,
    the committed fixture the tests read.
 
@@ -306,5 +306,5 @@ if __name__ == "__main__":
             raise SystemExit("prepare needs the reference's cuda_version directory")
         prepare(sys.argv[2])
     else:
-        path = sys.argv[2] if len(sys.argv) > 2 else os.path.join(ROOT, "gpurun_out", "ref_device_out.npz")
+        path = sys.argv[2] if len(sys.argv) > 2 else os.path.join(ROOT, "oracle", "_ref", "ref_device_out.npz")
         run(path) if step == "run" else finish(path)

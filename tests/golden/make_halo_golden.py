@@ -13,7 +13,7 @@ Three steps, as for make_device_golden.py:
 2. ``run [out.npz]`` (on the GPU machine; numpy and the CUDA driver only):
    uploads the constants copyConstants / set_cosmology / initHalomodel upload
    (bispectrum.cu:90-219, halomodel.cu:18-29), runs ref_halo_los and writes
-   the outputs (default gpurun_out/ref_halo_out.npz).
+   the outputs (default oracle/_ref/ref_halo_out.npz).
 3. ``finish [out.npz]``: merges inputs and outputs into
    tests/golden/reference_halo.npz, the committed fixture the tests read.
 """
@@ -121,5 +121,5 @@ if __name__ == "__main__":
             raise SystemExit("prepare needs the reference's cuda_version directory")
         prepare(sys.argv[2])
     else:
-        path = sys.argv[2] if len(sys.argv) > 2 else os.path.join(ROOT, "gpurun_out", "ref_halo_out.npz")
+        path = sys.argv[2] if len(sys.argv) > 2 else os.path.join(ROOT, "oracle", "_ref", "ref_halo_out.npz")
         run(path) if step == "run" else finish(path)
