@@ -348,7 +348,8 @@ struct GammaPolicy {
   __device__ __forceinline__ bool geometry(double phi, double psi, Geo& G) const {
     double c, s;
     if constexpr (sizeof(R) == 4) {  // on the integer pipe, for arguments in [0, 8)
-      if (!(psi >= 0 && psi < 8 && phi >= 0 && phi < 16)) return false;
+      // (by the high words: no FP64 instructions; negative numbers and NaN fail)
+      if ((uint32_t)__double2hiint(psi) >= 0x40200000u || (uint32_t)__double2hiint(phi) >= 0x40300000u) return false;
       int64_t qs, qc;
       i64_sincos(psi, d_i64sin, qs, qc);
       G.sp = i64_q62(qs), G.cp = i64_q62(qc);
@@ -435,7 +436,8 @@ struct GammaPolicy {
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const double A2 = G.A2[j], kap = G.k2[j] / A2;
-      same = same && kap < 1e3 && A2 > 1e-60 && A2 < 1e60 && G.mag[j] > 1e-30;  // (cre, cim normal floats)
+      same = same && kap < 1e3 && A2 > 1e-60 && A2 < 1e60 &&
+             (uint32_t)__double2hiint(G.mag[j]) > 0x39c00000u;  // 2^-99: cre, cim normal floats
       const int m = 128 + (int)(64 * fmin(kap, 1e3) + 16 * fmin(ib2, 1e4));
       const int64_t la = i64_log2(A2, d_i64tab) / 2;  // log2 A_j, Q57
       const double l2 = (double)la * 0x1p-57, ia = sf_to(i64_exp2(-(la >> 5), d_i64tab.ex2));

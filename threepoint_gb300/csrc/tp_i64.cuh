@@ -331,7 +331,7 @@ TP_HD bool i64_rounds_alike(double v, int ulps) {
 // no value is further than 2^28 units from the middle of two floats, so a larger
 // bound is never met (and its shift would leave 32 bits)
 TP_HD bool i64_rounds_alike(double v, double scale, int ulps) {
-  const int e = (int)(i64_bits(scale) >> 52 & 2047) - (int)(i64_bits(v) >> 52 & 2047) + 1, de = e > 0 ? e : 0;
+  const int e = ((int)(i64_bits(scale) >> 32) >> 20 & 2047) - ((int)(i64_bits(v) >> 32) >> 20 & 2047) + 1, de = e > 0 ? e : 0;
   return de < 20 && ulps < (0x10000000 >> de) && i64_rounds_alike(v, ulps << de);
 }
 
