@@ -655,11 +655,12 @@ cudaError_t launch_map3(const Map3Launch& L, int grid, size_t smem, char* scratc
                                 : launch_map3_t<float>(L, grid, smem, scratch, st);
 }
 
-// Below BK_SMALL points eight a block, else 32. Host call in us, 8 / 32 a block:
-// integer form 57 / 97 (8 points), 73 / 102 (2048), 113 / 107 (4096); FP64
-// instructions of a tabulated P(k) 150 / 415 (8), 268 / 428 (2048), 501 / 434
-// (4096). A warp a point: 91 us of FP64 instructions for one point, 155 else.
-constexpr long BK_SMALL = 3584;
+// Up to BK_SMALL points eight a block, which then are one wave (two CTAs on each
+// of 152 SMs), else 32. Host call in us, 8 / 32 a block: integer form 57 / 97 (8
+// points), 73 / 102 (2048), 113 / 107 (4096); FP64 instructions of a tabulated
+// P(k) 150 / 415 (8), 268 / 428 (2048), 501 / 434 (4096). A warp a point: 91 us
+// of FP64 instructions for one point, 155 else.
+constexpr long BK_SMALL = 8 * 2 * 152;
 
 cudaError_t launch_bkappa_points(int precision, const int* cosmo_idx, const double* ell, long n, const void* ncoef,
                                  const double* wscale, const void* ck, double* out, cudaStream_t st) {
@@ -668,7 +669,7 @@ cudaError_t launch_bkappa_points(int precision, const int* cosmo_idx, const doub
     if (n < 8)
       k_bkappa_points_f64<8, true><<<1, BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
                                                         (const CosmoK<double>*)ck, out);
-    else if (n < BK_SMALL)
+    else if (n <= BK_SMALL)
       k_bkappa_points_f64<8, false><<<(unsigned)((n + 7) / 8), BK_NT, 0, st>>>(cosmo_idx, ell, n, (const double*)ncoef, wscale,
                                                                         (const CosmoK<double>*)ck, out);
     else
