@@ -371,9 +371,9 @@ int tp_ctx_set_cov_tolerance(tp_ctx* ctx, int term, double rel_tol);
 int tp_ctx_set_halo_cluster(tp_ctx* ctx, int ctas);
 
 /* <Map^3> calls (tp_map3_batch, tp_map3_jobs_device) with no more integrals
- * than the device has CTA slots run one 8-CTA cluster per integral when on
- * (1, default); 2 uses clusters for every batch, 0 one CTA per integral
- * always. Same results bit for bit. */
+ * than the device has CTA slots run one cluster per integral when on (1,
+ * default): of 16 CTAs where all integrals fit the slots that way, else of 8; 2
+ * uses 8-CTA clusters for every batch, 0 one CTA per integral always. Same results bit for bit. */
 int tp_ctx_set_map3_cluster(tp_ctx* ctx, int on);
 
 /* The integrands that have a fast form beside their reference form (FP64: 64-bit
@@ -459,7 +459,8 @@ int tp_mlp_set_wait_limit(tp_mlp* m, int iterations);
 void* tp_mlp_stream(const tp_mlp* m);
 /* C = A B^T on the tensor cores (device pointers, the network's stream): A
  * [M][lda], B [N][ldb] BF16 with K contiguous, C [M][ldc] FP32; M % 128 == 0,
- * N % 32 == 0 with 32 <= N <= 256, K % 64 == 0, lda and ldb multiples of 8 */
+ * N % 32 == 0 with 32 <= N <= 256, K % 64 == 0, lda and ldb multiples of 8,
+ * A and B 16-byte aligned (TP_ERR_ARG otherwise) */
 int tp_gemm_bf16_device(tp_mlp* m, const void* A, int lda, const void* B, int ldb, float* C, int ldc, int M, int N,
                         int K);
 

@@ -55,3 +55,22 @@ def test_an_expired_wait_of_a_training_step():
         net.sync()
     finally:
         net.close()
+
+
+def test_misaligned_operands_are_refused():
+    """before a launch that would copy them in 16-byte pieces"""
+    import threepoint_gb300 as tp
+    import torch
+
+    a = torch.zeros(128 * 64 + 8, dtype=torch.bfloat16, device="cuda")
+    b = torch.zeros(32 * 64 + 8, dtype=torch.bfloat16, device="cuda")
+    c = torch.zeros((128, 32), device="cuda")
+    net = tp.MLP(max_batch=128)
+    try:
+        for i, j in ((1, 0), (0, 4), (3, 2)):
+            with pytest.raises(tp.ThreepointError) as e:
+                net.gemm_device(a[i:i + 128 * 64].view(128, 64), b[j:j + 32 * 64].view(32, 64), c)
+            assert e.value.status == tp.TP_ERR_ARG
+        net.gemm_device(a[8:].view(128, 64), b[8:].view(32, 64), c)
+    finally:
+        net.close()

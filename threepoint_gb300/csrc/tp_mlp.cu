@@ -1105,6 +1105,8 @@ extern "C" void* tp_mlp_stream(const tp_mlp* m) { return m ? (void*)m->stream : 
 extern "C" int tp_gemm_bf16_device(tp_mlp* m, const void* A, int lda, const void* B, int ldb, float* C, int ldc,
                                    int M, int N, int K) {
   if (!m || !A || !B || !C || lda % 8 || ldb % 8 || lda < K || ldb < K || ldc < N) return TP_ERR_ARG;
+  if (((uintptr_t)A | (uintptr_t)B) % 16 || (uintptr_t)C % 4)
+    return mlp_fail(m, TP_ERR_ARG, "gemm: A and B must be 16-byte aligned");  // copied in 16-byte pieces
   cudaSetDevice(m->device);
   GemmArgs g = gemm_args((const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb, M, N, K);
   g.flags = EPI_STORE_F32;
