@@ -539,8 +539,8 @@ class Context:
         _check(self._h, lib().tp_ctx_set_cov_tolerance(self._h, term, rel_tol))
 
     def set_map3_cluster(self, on=True):
-        """<Map^3> batches with no more integrals than CTA slots: one 8-CTA
-        cluster per integral (on) or one CTA (off); 2: clusters for every batch."""
+        """<Map^3> batches with no more integrals than CTA slots: one 16- or 8-CTA
+        cluster per integral (on) or one CTA (off); 2: 8-CTA clusters for every batch."""
         _check(self._h, lib().tp_ctx_set_map3_cluster(self._h, 2 if on == 2 else int(bool(on))))
 
     def set_reference_forms(self, on=True):

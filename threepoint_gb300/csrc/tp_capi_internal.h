@@ -64,8 +64,8 @@ struct tp_ctx {
   // CTAs that share one T5-T7 integral (a thread-block cluster): 16 (16 when
   // the batch leaves room for that many per integral, else 8), 8 or 1
   int halo_cluster = 16;
-  // <Map^3> host calls with no more integrals than CTA slots run one 8-CTA
-  // cluster per integral (0: always one CTA per integral)
+  // <Map^3> host calls with no more integrals than CTA slots run one 16- or
+  // 8-CTA cluster per integral (0: always one CTA per integral)
   int map3_cluster = 1;
   // the integrands' reference forms alone (tp_ctx_set_reference_forms)
   int reference_forms = 0;
