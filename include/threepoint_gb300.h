@@ -243,7 +243,10 @@ int tp_map3_jobs_device(tp_ctx* ctx, const int* job_cosmo_device, const double* 
  * device looks up the array's device address (cudaGetSymbolAddress): make it
  * before any stream capture. All calls share the array, so calls that overlap
  * on the GPU race; serialise them. Inputs, outputs and the context's
- * cosmology tables are the caller's/the context's, as in tp_map3_jobs_device. */
+ * cosmology tables are the caller's/the context's, as in tp_map3_jobs_device.
+ * In FP64 it uses the integer-arithmetic tables that are there (sets of up to 24
+ * cosmologies, or after another FP64 call of the context), else FP64
+ * instructions: the same integrals to rounding, several times slower. */
 int tp_map3_jobs_noalloc(tp_ctx* ctx, const int* job_cosmo_device, const double* job_theta_device, int n_jobs,
                          double phi_min, double phi_max, double l_min, double l_max, double rel_tol, int precision,
                          double* out_device, double* err_device, int* status_device);

@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(CNT) k_chi2(const double* xt, const double* da
 #pragma unroll 16
     for (; k0 < (i & ~31); ++k0) z = fma(xt[(size_t)k0 * n + i], r[k0], z);
     // a warp's rows end in the same block of 32: its loads go out together
-    // (past the diagonal they are not used)
+    // (past the diagonal they are not used; 64 models of 700 values 141 -> 127 us
+    // a host call against a row's last loads one after another)
     for (int h = 0; h < 2; ++h, k0 += 16) {
       double a[16];
 #pragma unroll
